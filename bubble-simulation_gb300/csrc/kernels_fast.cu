@@ -42,8 +42,8 @@ int batch_max_grid(bool fast, int ty) {
     return 0;
 }
 size_t batch_smem_bytes(int ty) {
-    return ty == 16 ? dev::ColumnLayout<float, 16, dev::kBatchShared<16>>::bytes
-                    : dev::ColumnLayout<float, 8, dev::kBatchShared<8>>::bytes;
+    return ty == 16 ? dev::BatchLayout<true, 16>::bytes
+                    : dev::BatchLayout<true, 8>::bytes;
 }
 cudaError_t batch_launch(bool fast, int ty, const void *lat, int n_lat, int n_items, int steps,
                          unsigned int *counters, int *status, int grid, unsigned int barrier_extra,

@@ -11,6 +11,7 @@
 #include "kernels.cuh"
 #include "launch.h"
 #include "stage_column.cuh"
+#include "stage_pair.cuh"
 
 namespace bubble {
 namespace launch_detail {
@@ -100,7 +101,21 @@ cudaError_t stage_column(const StageArgs<R> &A, const LatticeParams<R> &P, int l
     return cudaGetLastError();
 }
 
-// Whether a 16 x 16 FP32 stage launch takes the shared form: on request, or
+// A stage launch in the pair form (stage_pair.cuh).
+template <int FORM>
+cudaError_t stage_pair(const StageArgs<float> &A, const LatticeParams<float> &P, int lz, const StageMaps &maps,
+                       int tma_ok, int *status, cudaStream_t s) {
+    using L = dev::PairLayout;
+    auto k = dev::pair_kernel<FORM>;
+    cudaError_t e = ensure_smem(k, L::bytes);
+    if (e != cudaSuccess) return e;
+    if (lz < 1) lz = 1;
+    const dim3 grid(((P.nx + 15) / 16) * ((P.ny + 15) / 16), (P.nz + lz - 1) / lz);
+    k<<<grid, L::NT, L::bytes, s>>>(A, P, lz, maps, tma_ok, status);
+    return cudaGetLastError();
+}
+
+// Whether a 16 x 16 FP32 launch of the column kernel takes the shared form: on request, or
 // (BUBBLE_STAGE_FORM_AUTO) when column_stage_cost (params.h) rates it cheaper
 // at this chunk.  Measured per step, register vs shared form: 128^3 (256
 // CTAs) 0.239 vs 0.261 ms, 256^3 (2048 CTAs) 1.549 vs 1.508 ms, 512^3 (4096
@@ -116,12 +131,18 @@ inline bool shared_form(const LatticeParams<float> &P, const TileShape &shape) {
     return column_stage_cost(nx, ny, nz, shape.lz, true, sms) < column_stage_cost(nx, ny, nz, shape.lz, false, sms);
 }
 
-// A 16 x 16 FP32 stage launch in the form shared_form() picks.
+// A 16 x 16 FP32 stage launch: the pair form for the fast bag forms (faster
+// than either column form at every size measured, 32^3 .. 512^3), else the
+// column form that shared_form() picks.
 template <bool FAST, int FORM>
 cudaError_t stage_column16(const StageArgs<float> &A, const LatticeParams<float> &P, const TileShape &shape,
                            const StageMaps &maps, int tma_ok, int *status, cudaStream_t s) {
-    if (shared_form(P, shape)) return stage_column<float, FAST, FORM, 16, true>(A, P, shape.lz, maps, tma_ok, status, s);
-    return stage_column<float, FAST, FORM, 16, false>(A, P, shape.lz, maps, tma_ok, status, s);
+    if constexpr (FAST && dev::kPairForm<FORM>)
+        return stage_pair<FORM>(A, P, shape.lz, maps, tma_ok, status, s);
+    else if (shared_form(P, shape))
+        return stage_column<float, FAST, FORM, 16, true>(A, P, shape.lz, maps, tma_ok, status, s);
+    else
+        return stage_column<float, FAST, FORM, 16, false>(A, P, shape.lz, maps, tma_ok, status, s);
 }
 
 template <typename R, int MIXED>
@@ -144,7 +165,7 @@ namespace launch_detail {
 
 template <bool FAST, int TY>
 int batch_max_grid() {
-    using L = dev::ColumnLayout<float, TY, dev::kBatchShared<TY>>;
+    using L = dev::BatchLayout<FAST, TY>;
     auto k = dev::batch_kernel<FAST, TY>;
     if (ensure_smem(k, L::bytes) != cudaSuccess) return 0;
     int dev = 0, sms = 0, per_sm = 0;
@@ -157,7 +178,7 @@ int batch_max_grid() {
 template <bool FAST, int TY>
 cudaError_t batch_launch(const void *lat, int n_lat, int n_items, int steps, unsigned int *counters,
                          int *status, int grid, unsigned int barrier_extra, int barrier_shift, cudaStream_t s) {
-    using L = dev::ColumnLayout<float, TY, dev::kBatchShared<TY>>;
+    using L = dev::BatchLayout<FAST, TY>;
     auto k = dev::batch_kernel<FAST, TY>;
     cudaError_t e = ensure_smem(k, L::bytes);
     if (e != cudaSuccess) return e;

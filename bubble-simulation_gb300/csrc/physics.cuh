@@ -69,8 +69,14 @@ BUBBLE_DEV float2 hi2(const V4<float> &v) { return make_float2(v.z, v.w); }
 BUBBLE_DEV V4<float> v4of(float2 a, float2 b) { return V4<float>{a.x, a.y, b.x, b.y}; }
 BUBBLE_DEV float2 bc2(float s) { return make_float2(s, s); }
 BUBBLE_DEV float2 p_add(float2 a, float2 b) { return __fadd2_rn(a, b); }
-// a - b as a + b * (-1): exact product, one rounding
-BUBBLE_DEV float2 p_sub(float2 a, float2 b) { return __ffma2_rn(b, bc2(-1.0f), a); }
+BUBBLE_DEV float2 p_sub(float2 a, float2 b) {
+    float2 r;
+    asm("{\n\t.reg .b64 x, y, z;\n\tmov.b64 x, {%2, %3};\n\tmov.b64 y, {%4, %5};\n\t"
+        "sub.rn.f32x2 z, x, y;\n\tmov.b64 {%0, %1}, z;\n\t}"
+        : "=f"(r.x), "=f"(r.y)
+        : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+    return r;
+}
 BUBBLE_DEV float2 p_mul(float2 a, float2 b) { return __fmul2_rn(a, b); }
 BUBBLE_DEV float2 p_fma(float2 a, float2 b, float2 c) { return __ffma2_rn(a, b, c); }
 // x^2 + y^2 + z^2 with fixed roundings (the FAST mode's contraction of it)

@@ -1,0 +1,219 @@
+// Device-side physics of two lattice cells at once (fast arithmetic, FP32).
+//
+// The fast bag forms (plain, MIXED, perturbation) of physics.cuh on pairs of
+// cells: every quantity is a float2 whose halves belong to two different
+// cells, so the paired FP32 instructions of sm_100+ (two IEEE operations per
+// issue slot) carry the whole solver, with no exchange between the halves.
+// The formulas are those of the shaders cited in physics.cuh; every rounding
+// is explicit, so each call site computes the same bits.
+//
+// The rarely needed parts -- primitive recovery above gamma = 3 (with the
+// FP64 recovery of the MIXED and perturbation forms and the |Z| cap) and the
+// velocity clamp of a face state -- are decided by one test per pair.
+#pragma once
+
+#include "physics.cuh"
+
+namespace bubble {
+namespace dev {
+
+// A 4-vector of each of two cells: component pairs.
+struct P4 {
+    float2 x, y, z, w;
+};
+
+BUBBLE_DEV P4 pair_of(const float4 &a, const float4 &b) {
+    return P4{make_float2(a.x, a.y), make_float2(a.z, a.w), make_float2(b.x, b.y), make_float2(b.z, b.w)};
+}
+BUBBLE_DEV float4 pair_a(const P4 &q) { return make_float4(q.x.x, q.x.y, q.y.x, q.y.y); }
+BUBBLE_DEV float4 pair_b(const P4 &q) { return make_float4(q.z.x, q.z.y, q.w.x, q.w.y); }
+
+BUBBLE_DEV float2 rcp2(float2 a) { return make_float2(rcp_approx(a.x), rcp_approx(a.y)); }
+BUBBLE_DEV float2 sqrt2(float2 a) { return make_float2(sqrt_approx(a.x), sqrt_approx(a.y)); }
+BUBBLE_DEV float2 max2(float2 a, float s) { return make_float2(fmaxf(a.x, s), fmaxf(a.y, s)); }
+BUBBLE_DEV float2 dot3_2(float2 x, float2 y, float2 z) { return p_fma(z, z, p_fma(y, y, p_mul(x, x))); }
+
+// min(|a|, |b|) with the product of the signs
+BUBBLE_DEV float min_xorsign(float a, float b) {
+    float r;
+    asm("min.xorsign.abs.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
+    return r;
+}
+
+// Half of the MC-limited slope (limit_slope): 0 unless dm and dp have one
+// sign, else min(|dm + dp| / 4, |dm|, |dp|) with it.  The signed minimum
+// min(|dm|, |dp|) sign(dm dp), floored at 0, is 0 exactly when the signs
+// differ, so no comparison is needed: three instructions per value.
+BUBBLE_DEV float half_slope(float dm, float dp, float quarter_sum) {
+    return min_xorsign(quarter_sum, fmaxf(min_xorsign(dm, dp), 0.0f));
+}
+BUBBLE_DEV float2 half_slope2(float2 qm, float2 q, float2 qp) {
+    const float2 dm = p_sub(q, qm), dp = p_sub(qp, q);
+    const float2 h = p_mul(p_add(dm, dp), bc2(0.25f));
+    return make_float2(half_slope(dm.x, dp.x, h.x), half_slope(dm.y, dp.y, h.y));
+}
+
+// The two face states of a pair along one axis (face_states<FAST>): lo = q -
+// s/2, hi = q + s/2, pressure floored; the velocity clamp is hll_pair's.
+BUBBLE_DEV void face_states_pair(const P4 &qm, const P4 &q, const P4 &qp, float p_floor, P4 &lo, P4 &hi) {
+    const float2 sx = half_slope2(qm.x, q.x, qp.x), sy = half_slope2(qm.y, q.y, qp.y);
+    const float2 sz = half_slope2(qm.z, q.z, qp.z), sw = half_slope2(qm.w, q.w, qp.w);
+    lo = P4{p_sub(q.x, sx), p_sub(q.y, sy), p_sub(q.z, sz), max2(p_sub(q.w, sw), p_floor)};
+    hi = P4{p_add(q.x, sx), p_add(q.y, sy), p_add(q.z, sz), max2(p_add(q.w, sw), p_floor)};
+}
+
+// ---------------------------------------------------------------------------
+//  Primitive recovery
+// ---------------------------------------------------------------------------
+// One cell through the scalar recovery (|Z| cap, FP64 above gamma = 3,
+// velocity clamp).  Out of line: rarely taken and long.
+template <int FORM>
+__device__ __noinline__ V4<float> recover_slow(V4<float> u, float e_floor, float z_max, float p_floor, float e_bg,
+                                               float p_bg) {
+    LatticeParams<float> P{};
+    P.e_floor = e_floor;
+    P.z_max = z_max;
+    P.p_floor = p_floor;
+    P.e_bg = e_bg;
+    P.p_bg = p_bg;
+    return recover_sanitised<float, true, FORM>(u, P, 0.0f, z_max * z_max);
+}
+
+// sanitise(recover(u)) of two cells in two parts, so independent work can be
+// scheduled between them: recover_pair evaluates both cells by the formulas
+// that hold below gamma = 3; recover_fix sends a cell whose |v|^2 came out
+// above 8/9 (gamma > 3) through the scalar recovery.  That covers every cell
+// whose |Z| exceeds z_max E: the cap leaves |v|^2 > 8/9, and without it the
+// result is larger still (p is floored when E^2 - Z^2 is not positive).
+template <int FORM>
+BUBBLE_DEV P4 recover_pair(const V4<float> &ua, const V4<float> &ub, const LatticeParams<float> &P) {
+    const float2 de = max2(make_float2(ua.x, ub.x), P.e_floor);
+    const float2 zx = make_float2(ua.y, ub.y), zy = make_float2(ua.z, ub.z), zz = make_float2(ua.w, ub.w);
+    const float2 z2 = dot3_2(zx, zy, zz);
+    const float2 e = FORM == kPert ? p_add(bc2(P.e_bg), de) : de;
+    const float2 sq = sqrt2(p_fma(p_mul(bc2(4.0f), e), e, p_mul(bc2(-3.0f), z2)));
+    float2 p, s;
+    if constexpr (FORM == kPert) {
+        const float2 t = p_mul(z2, rcp2(p_fma(bc2(2.0f), e, sq)));
+        p = max2(p_fma(de, bc2((float)(1.0 / 3.0)), p_mul(t, bc2(-1.0f))), P.p_floor);
+        s = p_add(p_add(e, bc2(P.p_bg)), p);
+    } else {
+        p = max2(p_mul(p_fma(e, e, p_mul(z2, bc2(-1.0f))), rcp2(p_add(e, sq))), P.p_floor);
+        s = p_add(e, p);
+    }
+    const float2 inv = rcp2(s);
+    return P4{p_mul(zx, inv), p_mul(zy, inv), p_mul(zz, inv), p};
+}
+template <int FORM>
+BUBBLE_DEV void recover_fix(P4 &q, const V4<float> *ua, const V4<float> *ub, const LatticeParams<float> &P) {
+    const float2 v2 = dot3_2(q.x, q.y, q.z);
+    constexpr float kFast = 8.0f / 9.0f;
+    if (fmaxf(v2.x, v2.y) > kFast) {
+        if (v2.x > kFast) {
+            const V4<float> r = recover_slow<FORM>(*ua, P.e_floor, P.z_max, P.p_floor, P.e_bg, P.p_bg);
+            q.x.x = r.x;
+            q.y.x = r.y;
+            q.z.x = r.z;
+            q.w.x = r.w;
+        }
+        if (v2.y > kFast) {
+            const V4<float> r = recover_slow<FORM>(*ub, P.e_floor, P.z_max, P.p_floor, P.e_bg, P.p_bg);
+            q.x.y = r.x;
+            q.y.y = r.y;
+            q.z.y = r.z;
+            q.w.y = r.w;
+        }
+    }
+}
+
+// ---------------------------------------------------------------------------
+//  HLL face flux of two faces along one axis
+// ---------------------------------------------------------------------------
+struct PairSide {
+    P4 u, f;         // conserved state and flux along the axis
+    float2 nlm, lp;  // minus the lower wave speed, the upper wave speed
+};
+
+// With c_s^2 = 1/3, D = 3 - v^2 and T = D - 2 vd^2 the wave speeds
+// (2 vd -+ sqrt((1 - v^2) T)) / D are those of face_side: numerator and
+// denominator scaled by 3.
+template <int AXIS, int FORM>
+BUBBLE_DEV PairSide pair_side(const P4 &q, float2 v2, const LatticeParams<float> &P) {
+    PairSide s;
+    const float2 vd = AXIS == 0 ? q.x : (AXIS == 1 ? q.y : q.z);
+    const float2 p = q.w;
+    const float2 om = p_sub(bc2(1.0f), v2);
+    const float2 pf = FORM == kPert ? p_add(bc2(P.p_bg), p) : p;  // the full pressure
+    const float2 w = p_mul(p_mul(bc2(4.0f), pf), rcp2(om));
+    s.u.x = FORM == kPert ? p_fma(w, v2, p_mul(bc2(3.0f), p)) : p_sub(w, p);
+    s.u.y = p_mul(w, q.x);
+    s.u.z = p_mul(w, q.y);
+    s.u.w = p_mul(w, q.z);
+    const float2 d = p_sub(bc2(3.0f), v2);
+    const float2 inv = rcp2(d);
+    const float2 tv = p_mul(vd, bc2(-2.0f));
+    const float2 sq = sqrt2(p_mul(om, p_fma(tv, vd, d)));
+    s.nlm = p_mul(p_add(sq, tv), inv);
+    s.lp = p_mul(p_sub(sq, tv), inv);
+    s.f.x = p_mul(w, vd);
+    s.f.y = AXIS == 0 ? p_fma(s.u.y, vd, p) : p_mul(s.u.y, vd);
+    s.f.z = AXIS == 1 ? p_fma(s.u.z, vd, p) : p_mul(s.u.z, vd);
+    s.f.w = AXIS == 2 ? p_fma(s.u.w, vd, p) : p_mul(s.u.w, vd);
+    return s;
+}
+
+// |v|^2 of a pair whose x and y components may be exchanged: the same bits
+// either way.
+BUBBLE_DEV float2 speed2(const P4 &q, bool exchanged) {
+    return dot3_2(exchanged ? q.y : q.x, exchanged ? q.x : q.y, q.z);
+}
+
+// The velocity half of sanitise on the halves of a pair beyond the cap.
+BUBBLE_DEV void clamp_pair(P4 &q, float2 &v2, float zmax2, bool exchanged) {
+    float2 f;
+    f.x = v2.x > zmax2 ? __fsqrt_rn(__fdiv_rn(zmax2, v2.x)) : 1.0f;
+    f.y = v2.y > zmax2 ? __fsqrt_rn(__fdiv_rn(zmax2, v2.y)) : 1.0f;
+    q.x = p_mul(q.x, f);
+    q.y = p_mul(q.y, f);
+    q.z = p_mul(q.z, f);
+    v2 = speed2(q, exchanged);
+    v2 = make_float2(fminf(v2.x, zmax2), fminf(v2.y, zmax2));
+}
+
+// One side of a face pair and its |v|^2.  `exchanged`: q holds (vy, vx, vz,
+// p), for a y face taken as AXIS 0; the flux is then (E, Zy, Zx, Zz) with the
+// bits of AXIS 1.
+struct FacePair {
+    P4 l, r;
+    float2 vl, vr;
+};
+BUBBLE_DEV FacePair face_pair(const P4 &l, const P4 &r, bool exchanged = false) {
+    return FacePair{l, r, speed2(l, exchanged), speed2(r, exchanged)};
+}
+BUBBLE_DEV float max_speed2(const FacePair &f) {
+    return fmaxf(fmaxf(f.vl.x, f.vl.y), fmaxf(f.vr.x, f.vr.y));
+}
+// The velocity clamps of a face pair one of whose speeds is beyond the cap.
+BUBBLE_DEV void clamp_face(FacePair &f, float zmax2, bool exchanged = false) {
+    clamp_pair(f.l, f.vl, zmax2, exchanged);
+    clamp_pair(f.r, f.vr, zmax2, exchanged);
+}
+
+template <int AXIS, int FORM>
+BUBBLE_DEV P4 hll_pair(const FacePair &f, const LatticeParams<float> &P) {
+    const PairSide L = pair_side<AXIS, FORM>(f.l, f.vl, P);
+    const PairSide R = pair_side<AXIS, FORM>(f.r, f.vr, P);
+    const float2 ns = make_float2(fmaxf(fmaxf(L.nlm.x, R.nlm.x), 0.0f), fmaxf(fmaxf(L.nlm.y, R.nlm.y), 0.0f));
+    const float2 sx = make_float2(fmaxf(fmaxf(L.lp.x, R.lp.x), 0.0f), fmaxf(fmaxf(L.lp.y, R.lp.y), 0.0f));
+    // (s_max f_L - s_min f_R + s_min s_max (u_R - u_L)) / (s_max - s_min)
+    const float2 inv = rcp2(p_add(ns, sx));
+    const float2 ca = p_mul(sx, inv), cb = p_mul(ns, inv);
+    const float2 cc = p_mul(ns, ca);
+    return P4{p_fma(ca, L.f.x, p_fma(cb, R.f.x, p_mul(cc, p_sub(L.u.x, R.u.x)))),
+              p_fma(ca, L.f.y, p_fma(cb, R.f.y, p_mul(cc, p_sub(L.u.y, R.u.y)))),
+              p_fma(ca, L.f.z, p_fma(cb, R.f.z, p_mul(cc, p_sub(L.u.z, R.u.z)))),
+              p_fma(ca, L.f.w, p_fma(cb, R.f.w, p_mul(cc, p_sub(L.u.w, R.u.w))))};
+}
+
+}  // namespace dev
+}  // namespace bubble

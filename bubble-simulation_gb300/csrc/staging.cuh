@@ -51,6 +51,7 @@ BUBBLE_DEV bool mbar_try_wait(uint64_t *bar, uint32_t parity) {
 // Bounded wait: gives up after 2^shift SM cycles (2^31 by default, about a
 // second at GB300 clocks).
 BUBBLE_DEV bool mbar_wait_bounded(uint64_t *bar, uint32_t parity, int shift) {
+    if (mbar_try_wait(bar, parity)) return true;
     const long long start = clock64();
     const long long limit = 1ll << shift;
     while (!mbar_try_wait(bar, parity)) {

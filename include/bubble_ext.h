@@ -29,8 +29,10 @@ int bubble_ext_set_path(bubble_sim *sim, int32_t path);
 int bubble_ext_set_tile(bubble_sim *sim, int32_t ty, int32_t lz);
 int bubble_ext_get_tile(const bubble_sim *sim, int32_t *ty, int32_t *lz);
 
-/* Form of the fused kernel for FP32 16 x 16 tiles; both forms give
- * identical bits.  REGISTERS keeps each column's z pipeline in registers
+/* Form of the fused column kernel for FP32 16 x 16 tiles; both forms give
+ * identical bits.  The fast arithmetic of the bag equation of state (SINGLE,
+ * MIXED, PERTURBATION) has one form of its own, two cells per thread, and
+ * runs it whatever is set here.  REGISTERS keeps each column's z pipeline in registers
  * (two CTAs per SM); SHARED reads it back from shared memory (three CTAs
  * per SM, faster once a launch fills more than one wave); AUTO (default)
  * takes the form a cost model of the launch rates cheaper for the lattice
