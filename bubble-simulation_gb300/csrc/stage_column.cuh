@@ -552,6 +552,7 @@ __global__ void __launch_bounds__(ColumnLayout<R, TY, LEAN>::NT, ColumnLayout<R,
     stage_kernel(StageArgs<R> A, LatticeParams<R> P, int lz, const __grid_constant__ StageMaps maps,
                     int tma_ok, int *status) {
     extern __shared__ __align__(128) unsigned char smem[];
+    await_previous_launch();
     column_item<R, FAST, FORM, TY, LEAN>(smem, A, P, lz, &maps, tma_ok, status, blockIdx.x, blockIdx.y);
 }
 

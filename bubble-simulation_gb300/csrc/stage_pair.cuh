@@ -523,6 +523,7 @@ __global__ void __launch_bounds__(PairLayout::NT, PairLayout::MIN_BLOCKS)
     pair_kernel(StageArgs<float> A, LatticeParams<float> P, int lz, const __grid_constant__ StageMaps maps, int tma_ok,
                 int *status) {
     extern __shared__ __align__(128) unsigned char smem[];
+    await_previous_launch();
     pair_item<FORM>(smem, A, P, lz, &maps, tma_ok, status, blockIdx.x, blockIdx.y);
 }
 

@@ -72,3 +72,32 @@ def test_pair_form(bubble, oracle_mod, gpu, grid, precision):
     for lz in (1, 3, grid[2]):
         got = _run(bubble, grid, f0, u0, precision, "fast", lz)
         assert np.array_equal(got[0], fast[0]) and np.array_equal(got[1], fast[1]), lz
+
+
+@pytest.mark.parametrize("precision,math", [("mixed", "fast"), ("single", "strict")])
+def test_step_under_capture(bubble, oracle_mod, gpu, precision, math):
+    """A step recorded into a CUDA graph (plain launches there, dependent ones
+    outside) and replayed gives the bits of a step launched directly."""
+    import torch
+
+    grid = (50, 48, 20)
+    f0, u0, _ = _state(oracle_mod, grid, "single")
+    spec = bubble.SimulationSpec(grid=grid, bubbles=0, nucleation="centre", precision=precision, math=math)
+    with bubble.Simulation(spec) as sim:
+        sim.load_state(f0, u0)
+        sim.advance(2)
+        want = sim.copy_state()
+    stream = torch.cuda.Stream()
+    with bubble.Simulation(spec) as sim:
+        sim.set_stream(stream.cuda_stream)
+        sim.load_state(f0, u0)
+        sim.advance(1)
+        sim.synchronize()
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=stream):
+            sim.record_steps(1)
+        graph.replay()
+        torch.cuda.synchronize()
+        got = sim.copy_state()
+        sim.set_stream(None)
+    assert np.array_equal(got[0], want[0]) and np.array_equal(got[1], want[1])
