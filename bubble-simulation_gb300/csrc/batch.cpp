@@ -294,6 +294,7 @@ int Batch::add(const bubble_spec &spec, uint32_t *index, std::string &err) {
         L.solo = tiles * (((long)L.grid[2] + 31) / 32) >= 2L * std::max(sms, 1);
         if (L.solo) {
             L.lz = default_chunk(L.grid, ty_, true);
+            if (ty_ == 16) L.pair_lz = pair_chunk(L.grid);
         } else {
             // equal chunks no longer than the cap
             const int nz = (int)L.grid[2];
@@ -633,7 +634,8 @@ int Batch::launch_solo(Lat &L, uint64_t k, std::string &err) {
             A.a1 = kRK3[st][1];
             A.dt = L.dt;
             A.stage = st;
-            const TileShape tile{tile_x_for(ty_), ty_, L.lz};
+            TileShape tile{tile_x_for(ty_), ty_, L.lz};
+            tile.pair_lz = L.pair_lz;
             const int tma = L.tma_ok ? 1 : 0;
             const cudaError_t e =
                 fast_ ? launch::stage_f32_fast(A, L.P, tile, 0, L.maps[in[st]], tma, d_status_, stream_)

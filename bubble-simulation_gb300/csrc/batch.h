@@ -73,6 +73,7 @@ class Batch {
         uint64_t steps = 0;
         uint32_t cur = 0;
         int lz = 16;
+        int pair_lz = 0;  // of a solo lattice: TileShape::pair_lz
         // A lattice that fills the GPU by itself (two CTAs per SM with
         // 32-plane chunks) gains nothing from the shared launch: it runs
         // through the plain stage kernel with the plain path's chunk.

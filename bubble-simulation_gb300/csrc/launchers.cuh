@@ -162,7 +162,7 @@ template <bool FAST, int FORM>
 cudaError_t stage_column16(const StageArgs<float> &A, const LatticeParams<float> &P, const TileShape &shape,
                            const StageMaps &maps, int tma_ok, int *status, cudaStream_t s) {
     if constexpr (FAST && dev::kPairForm<FORM>)
-        return stage_pair<FORM>(A, P, shape.lz, maps, tma_ok, status, s);
+        return stage_pair<FORM>(A, P, shape.pair_lz > 0 ? shape.pair_lz : shape.lz, maps, tma_ok, status, s);
     else if (shared_form(P, shape))
         return stage_column<float, FAST, FORM, 16, true>(A, P, shape.lz, maps, tma_ok, status, s);
     else

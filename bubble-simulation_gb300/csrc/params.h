@@ -78,7 +78,8 @@ struct DiagResult {
 // Tile shape of the fused stage kernel.
 struct TileShape {
     int32_t tx, ty, lz;  // x, y tile (cells) and z chunk (planes)
-    int32_t form = 0;    // BUBBLE_STAGE_FORM_* of 16 x 16 FP32 launches
+    int32_t form = 0;    // BUBBLE_STAGE_FORM_* of 16 x 16 FP32 launches of the column kernel
+    int32_t pair_lz = 0; // z chunk of the pair form where lz was not set by the caller; 0: lz
 };
 
 // The stage kernel's tiles are 16 x 16 (FP32 default: the least perimeter,
@@ -108,6 +109,33 @@ inline double column_stage_cost(uint32_t nx, uint32_t ny, uint32_t nz, int lz, b
     const long last = m - (rounds - 1) * k;
     const double p_last = last == k ? p : (last == 1 ? 0.65 * p : 0.8 * p);
     return ((double)(rounds - 1) * p + p_last) * (double)(lz_eff + 2);
+}
+
+// Cost model of one stage launch in the pair form, in plane times of a CTA
+// that shares its SM with two others (2.5 us on GB300).  Three CTAs fit on an
+// SM; a plane takes 0.57 with one there, 0.77 with two.  A chunk costs its
+// planes plus 1.6 for its two lighter warm-up planes and its start, a launch
+// 0.64.  A launch of one wave runs at the pace of its fullest SM; beyond one
+// wave CTAs are handed out as they finish, so the time lies between the busiest
+// SM's rounds and the even share (weighted 0.8 and 0.2).  Against the measured
+// step times of cubes from 32^3 to 384^3 over 20 chunk lengths the cheapest
+// pick is the fastest or within 3.6 % of it (176^3; 1 % at the others); the
+// column kernel's chunk is up to 1.7x off on small ones (us per step, that
+// chunk and the pick: 32^3 29.9 17.5, 48^3 30.6 23.2, 96^3 84.1 76.6, 160^3
+// 328 304).
+inline double pair_stage_cost(uint32_t nx, uint32_t ny, uint32_t nz, int lz, int sms) {
+    if (lz < 1) lz = 1;
+    if (sms < 1) sms = 1;
+    const long tiles = (long)((nx + 15) / 16) * (long)((ny + 15) / 16);
+    const long chunks = ((long)nz + lz - 1) / lz;
+    const long lz_eff = ((long)nz + chunks - 1) / chunks;
+    const long ctas = tiles * chunks;
+    const long m = (ctas + sms - 1) / sms;
+    const long full = (m - 1) / 3, last = m - 3 * full;
+    const double rounds = (double)full + (last == 1 ? 0.57 : (last == 2 ? 0.77 : 1.0));
+    const double share = (double)ctas / (3.0 * sms);
+    const double waves = share <= 1.0 ? rounds : 0.8 * rounds + 0.2 * share;
+    return waves * ((double)lz_eff + 1.6) + 0.64;
 }
 
 }  // namespace bubble

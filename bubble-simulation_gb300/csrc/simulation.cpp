@@ -105,6 +105,23 @@ int default_chunk(const uint32_t grid[3], int ty, bool fp32) {
     return (int)lz;
 }
 
+int pair_chunk(const uint32_t grid[3]) {
+    int dev = 0, sms = 148;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    double best = 1e300;
+    int best_lz = (int)grid[2];
+    for (int chunks = 1; chunks <= (int)grid[2]; ++chunks) {  // ties go to longer chunks
+        const int lz = ((int)grid[2] + chunks - 1) / chunks;
+        const double c = pair_stage_cost(grid[0], grid[1], grid[2], lz, sms);
+        if (c < best * (1.0 - 1e-9)) {
+            best = c;
+            best_lz = lz;
+        }
+    }
+    return best_lz;
+}
+
 int Simulation::create(const bubble_spec &spec, std::unique_ptr<Simulation> &out, std::string &err) {
     const std::string msg = validate_model(spec.model);
     if (!msg.empty()) {
@@ -148,6 +165,7 @@ int Simulation::create(const bubble_spec &spec, std::unique_ptr<Simulation> &out
     sim->tile_.ty = 16;
     sim->tile_.tx = tile_x_for(sim->tile_.ty);
     sim->tile_.lz = default_chunk(sim->grid_, sim->tile_.ty, !sim->is_f64());
+    sim->tile_.pair_lz = pair_chunk(sim->grid_);
     BUBBLE_CUDA(cudaStreamCreateWithFlags(&sim->stream_, cudaStreamNonBlocking), "cudaStreamCreate");
     sim->own_stream_ = true;
     int rc = sim->allocate(err);
@@ -368,6 +386,7 @@ int Simulation::resize(const uint32_t grid[3], std::string &err) {
     spec_.grid[2] = grid[2];
     n_cells_ = (uint64_t)grid[0] * grid[1] * grid[2];
     tile_.lz = default_chunk(grid_, tile_.ty, !is_f64());
+    tile_.pair_lz = pair_chunk(grid_);
     int rc = allocate(err);
     if (rc != BUBBLE_OK) return rc;
     const Derived d = derive(spec_.model);

@@ -171,6 +171,9 @@ int arith_mode(const bubble_spec &spec);
 // otherwise enough CTAs to fill the GPU while keeping each chunk's warm-up a
 // small fraction of its work.
 int default_chunk(const uint32_t grid[3], int ty, bool fp32);
+// z chunk of the pair form (stage_pair.cuh) where the caller set none: the
+// cheapest under pair_stage_cost (params.h).
+int pair_chunk(const uint32_t grid[3]);
 
 // Test hook: make the next device allocation of this process fail.
 void inject_allocation_failure();

@@ -25,7 +25,9 @@ int bubble_ext_set_path(bubble_sim *sim, int32_t path);
 /* Tile of the fused kernel: y extent, which fixes the x extent (FP32: 16
  * for 16 x 16 tiles, the default, in every form; 8 for 32 x 8 in the plain
  * and MIXED forms; 4 for 32 x 4 in those forms with the fast arithmetic;
- * FP64: 16 (default) or 4 for 32 x 4) and z chunk (planes marched per CTA). */
+ * FP64: 16 (default) or 4 for 32 x 4) and z chunk (planes marched per CTA).
+ * Until it is set, the fast bag forms pick a chunk of their own and the chunk
+ * reported is the column kernel's. */
 int bubble_ext_set_tile(bubble_sim *sim, int32_t ty, int32_t lz);
 int bubble_ext_get_tile(const bubble_sim *sim, int32_t *ty, int32_t *lz);
 
