@@ -155,7 +155,7 @@ inline bool shared_form(const LatticeParams<float> &P, const TileShape &shape) {
     return column_stage_cost(nx, ny, nz, shape.lz, true, sms) < column_stage_cost(nx, ny, nz, shape.lz, false, sms);
 }
 
-// A 16 x 16 FP32 stage launch: the pair form for the fast bag forms (faster
+// A 16 x 16 FP32 stage launch: the pair form for the fast forms it has (faster
 // than either column form at every size measured, 32^3 .. 512^3), else the
 // column form that shared_form() picks.
 template <bool FAST, int FORM>

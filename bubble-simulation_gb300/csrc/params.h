@@ -37,8 +37,9 @@ struct LatticeParams {
     // floors unshifted, for the other forms.
     R e_bg, p_bg;
     // Gamma-law equation of state: c_s^2 = Gamma - 1 and the offset e0 of
-    // e = p / (Gamma - 1) + e0; both 0 for the bag model.
-    R eos_c2, eos_e0;
+    // e = p / (Gamma - 1) + e0; both 0 for the bag model.  eos_k = 1 / c_s^2 + 1
+    // (the enthalpy is eos_k p + e0) and eos_cs = c_s, for the fast arithmetic.
+    R eos_c2, eos_e0, eos_k, eos_cs;
     // Thermal potential V(phi) + gamma/2 (T^2 - T_ref^2) phi^2 - A/3 (T - T_ref) phi^3:
     // th_k = a/3, th_g = gamma, th_h = A/3, th_a = A, th_lo = sqrt(3 gamma / (4 a))
     // (the physical branch is T >= th_lo |phi|), th_i2a = 1/(2a), the radiation

@@ -1,7 +1,7 @@
 // Device-side physics of two lattice cells at once (fast arithmetic, FP32).
 //
-// The fast bag forms (plain, MIXED, perturbation) of physics.cuh on pairs of
-// cells: every quantity is a float2 whose halves belong to two different
+// The fast bag forms (plain, MIXED, perturbation) and the fast gamma law of
+// physics.cuh on pairs of cells: every quantity is a float2 whose halves belong to two different
 // cells, so the paired FP32 instructions of sm_100+ (two IEEE operations per
 // issue slot) carry the whole solver, with no exchange between the halves.
 // The formulas are those of the shaders cited in physics.cuh; every rounding
@@ -67,15 +67,21 @@ BUBBLE_DEV void face_states_pair(const P4 &qm, const P4 &q, const P4 &qp, float 
 // ---------------------------------------------------------------------------
 // One cell through the scalar recovery (|Z| cap, FP64 above gamma = 3,
 // velocity clamp).  Out of line: rarely taken and long.
+// c0, c1 are e_bg and p_bg, or eos_c2 and eos_e0 of the gamma law.
 template <int FORM>
-__device__ __noinline__ V4<float> recover_slow(V4<float> u, float e_floor, float z_max, float p_floor, float e_bg,
-                                               float p_bg) {
+__device__ __noinline__ V4<float> recover_slow(V4<float> u, float e_floor, float z_max, float p_floor, float c0,
+                                               float c1) {
     LatticeParams<float> P{};
     P.e_floor = e_floor;
     P.z_max = z_max;
     P.p_floor = p_floor;
-    P.e_bg = e_bg;
-    P.p_bg = p_bg;
+    if constexpr (FORM == kGamma) {
+        P.eos_c2 = c0;
+        P.eos_e0 = c1;
+    } else {
+        P.e_bg = c0;
+        P.p_bg = c1;
+    }
     return recover_sanitised<float, true, FORM>(u, P, 0.0f, z_max * z_max);
 }
 
@@ -90,6 +96,19 @@ BUBBLE_DEV P4 recover_pair(const V4<float> &ua, const V4<float> &ub, const Latti
     const float2 de = max2(make_float2(ua.x, ub.x), P.e_floor);
     const float2 zx = make_float2(ua.y, ub.y), zy = make_float2(ua.z, ub.z), zz = make_float2(ua.w, ub.w);
     const float2 z2 = dot3_2(zx, zy, zz);
+    if constexpr (FORM == kGamma) {
+        // with s = E + p the closure is s^2 - B s + c2 Z^2 = 0, B = E + c2 (E -
+        // e0), whose larger root the Newton steps of prim_from_cons_gamma
+        // approach; p = c2 (E - e0 - Z^2 / s) keeps p's digits.  No real root
+        // (NaN) and a root below the floor both end at the floor.
+        const float2 x = p_sub(de, bc2(P.eos_e0));
+        const float2 b = p_fma(bc2(P.eos_c2), x, de);
+        const float2 sq = sqrt2(p_fma(b, b, p_mul(bc2(-4.0f * P.eos_c2), z2)));
+        const float2 s = p_mul(bc2(0.5f), p_add(b, sq));
+        const float2 p = max2(p_mul(bc2(P.eos_c2), p_sub(x, p_mul(z2, rcp2(s)))), P.p_floor);
+        const float2 inv = rcp2(p_add(de, p));
+        return P4{p_mul(zx, inv), p_mul(zy, inv), p_mul(zz, inv), p};
+    }
     const float2 e = FORM == kPert ? p_add(bc2(P.e_bg), de) : de;
     const float2 sq = sqrt2(p_fma(p_mul(bc2(4.0f), e), e, p_mul(bc2(-3.0f), z2)));
     float2 p, s;
@@ -109,15 +128,16 @@ BUBBLE_DEV void recover_fix(P4 &q, const V4<float> *ua, const V4<float> *ub, con
     const float2 v2 = dot3_2(q.x, q.y, q.z);
     constexpr float kFast = 8.0f / 9.0f;
     if (fmaxf(v2.x, v2.y) > kFast) {
+        const float c0 = FORM == kGamma ? P.eos_c2 : P.e_bg, c1 = FORM == kGamma ? P.eos_e0 : P.p_bg;
         if (v2.x > kFast) {
-            const V4<float> r = recover_slow<FORM>(*ua, P.e_floor, P.z_max, P.p_floor, P.e_bg, P.p_bg);
+            const V4<float> r = recover_slow<FORM>(*ua, P.e_floor, P.z_max, P.p_floor, c0, c1);
             q.x.x = r.x;
             q.y.x = r.y;
             q.z.x = r.z;
             q.w.x = r.w;
         }
         if (v2.y > kFast) {
-            const V4<float> r = recover_slow<FORM>(*ub, P.e_floor, P.z_max, P.p_floor, P.e_bg, P.p_bg);
+            const V4<float> r = recover_slow<FORM>(*ub, P.e_floor, P.z_max, P.p_floor, c0, c1);
             q.x.y = r.x;
             q.y.y = r.y;
             q.z.y = r.z;
@@ -144,17 +164,27 @@ BUBBLE_DEV PairSide pair_side(const P4 &q, float2 v2, const LatticeParams<float>
     const float2 p = q.w;
     const float2 om = p_sub(bc2(1.0f), v2);
     const float2 pf = FORM == kPert ? p_add(bc2(P.p_bg), p) : p;  // the full pressure
-    const float2 w = p_mul(p_mul(bc2(4.0f), pf), rcp2(om));
+    const float2 w = p_mul(FORM == kGamma ? p_fma(bc2(P.eos_k), p, bc2(P.eos_e0)) : p_mul(bc2(4.0f), pf), rcp2(om));
     s.u.x = FORM == kPert ? p_fma(w, v2, p_mul(bc2(3.0f), p)) : p_sub(w, p);
     s.u.y = p_mul(w, q.x);
     s.u.z = p_mul(w, q.y);
     s.u.w = p_mul(w, q.z);
-    const float2 d = p_sub(bc2(3.0f), v2);
-    const float2 inv = rcp2(d);
-    const float2 tv = p_mul(vd, bc2(-2.0f));
-    const float2 sq = sqrt2(p_mul(om, p_fma(tv, vd, d)));
-    s.nlm = p_mul(p_add(sq, tv), inv);
-    s.lp = p_mul(p_sub(sq, tv), inv);
+    if constexpr (FORM == kGamma) {
+        // the same with c_s^2 = c2, unscaled: D = 1 - c2 v^2, T = D - (1 - c2) vd^2
+        const float2 d = p_fma(v2, bc2(-P.eos_c2), bc2(1.0f));
+        const float2 inv = rcp2(d);
+        const float2 tv = p_mul(vd, bc2(P.eos_c2 - 1.0f));
+        const float2 sq = p_mul(bc2(P.eos_cs), sqrt2(p_mul(om, p_fma(tv, vd, d))));
+        s.nlm = p_mul(p_add(sq, tv), inv);
+        s.lp = p_mul(p_sub(sq, tv), inv);
+    } else {
+        const float2 d = p_sub(bc2(3.0f), v2);
+        const float2 inv = rcp2(d);
+        const float2 tv = p_mul(vd, bc2(-2.0f));
+        const float2 sq = sqrt2(p_mul(om, p_fma(tv, vd, d)));
+        s.nlm = p_mul(p_add(sq, tv), inv);
+        s.lp = p_mul(p_sub(sq, tv), inv);
+    }
     s.f.x = p_mul(w, vd);
     s.f.y = AXIS == 0 ? p_fma(s.u.y, vd, p) : p_mul(s.u.y, vd);
     s.f.z = AXIS == 1 ? p_fma(s.u.z, vd, p) : p_mul(s.u.z, vd);

@@ -272,6 +272,8 @@ LatticeParams<float> lattice_params_f32(const bubble_spec &spec) {
     if (spec.eos == BUBBLE_EOS_GAMMA_LAW) {
         p.eos_c2 = spec.eos_param[0] - 1.0f;
         p.eos_e0 = spec.eos_param[1];
+        p.eos_k = (float)(1.0 / (double)p.eos_c2 + 1.0);
+        p.eos_cs = std::sqrt(p.eos_c2);
     }
     if (spec.eos == BUBBLE_EOS_THERMAL) {
         const float g = spec.eos_param[0], a = spec.eos_param[1];

@@ -35,8 +35,8 @@ def _state(oracle_mod, grid, kind):
     return f, u, float(o.d["e_ref"])
 
 
-def _run(bubble, grid, f0, u0, precision, math, lz=None):
-    spec = bubble.SimulationSpec(grid=grid, bubbles=0, nucleation="centre", precision=precision, math=math)
+def _run(bubble, grid, f0, u0, precision, math, lz=None, **kw):
+    spec = bubble.SimulationSpec(grid=grid, bubbles=0, nucleation="centre", precision=precision, math=math, **kw)
     with bubble.Simulation(spec) as sim:
         if lz is not None:
             sim.set_tile(16, lz)
@@ -71,6 +71,23 @@ def test_pair_form(bubble, oracle_mod, gpu, grid, precision):
         assert np.all(e_fast <= 2.0 * e_strict + 1e-6), (e_fast, e_strict)
     for lz in (1, 3, grid[2]):
         got = _run(bubble, grid, f0, u0, precision, "fast", lz)
+        assert np.array_equal(got[0], fast[0]) and np.array_equal(got[1], fast[1]), lz
+
+
+@pytest.mark.parametrize("eos_param", [(1.2, 0.05), (2.0, 0.0), (1.02, 0.12)])
+@pytest.mark.parametrize("grid", GRIDS)
+def test_pair_form_gamma_law(bubble, oracle_mod, gpu, grid, eos_param):
+    """The gamma law's pair form (closed-form recovery) against the strict form
+    (eight Newton steps): the fast arithmetic's bar of 1e-5 per component, and
+    the same bits for every chunking."""
+    f0, u0, _ = _state(oracle_mod, grid, "single")
+    kw = dict(eos="gamma_law", eos_param=eos_param)
+    strict = _run(bubble, grid, f0, u0, "single", "strict", **kw)
+    fast = _run(bubble, grid, f0, u0, "single", "fast", **kw)
+    for a, s in zip(fast, strict):
+        assert np.isfinite(a).all() and np.all(_err(a, s) <= 1e-5), _err(a, s)
+    for lz in (1, 3, grid[2]):
+        got = _run(bubble, grid, f0, u0, "single", "fast", lz, **kw)
         assert np.array_equal(got[0], fast[0]) and np.array_equal(got[1], fast[1]), lz
 
 
