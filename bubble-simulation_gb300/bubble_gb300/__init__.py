@@ -219,8 +219,7 @@ class Simulation:
     def set_stage_form(self, form: str):
         """Form of the fused kernel for FP32 16 x 16 tiles: "auto" (default),
         "registers" or "shared" (identical bits; include/bubble_ext.h).  The
-        fast bag forms and the fast gamma law have one form and run it
-        whatever is set."""
+        fast arithmetic has one form and runs it whatever is set."""
         check(self._L.bubble_ext_set_stage_form(self._h, _lib.STAGE_FORMS[form]))
 
     def tile(self) -> tuple[int, int]:

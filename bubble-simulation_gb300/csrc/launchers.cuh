@@ -155,13 +155,13 @@ inline bool shared_form(const LatticeParams<float> &P, const TileShape &shape) {
     return column_stage_cost(nx, ny, nz, shape.lz, true, sms) < column_stage_cost(nx, ny, nz, shape.lz, false, sms);
 }
 
-// A 16 x 16 FP32 stage launch: the pair form for the fast forms it has (faster
+// A 16 x 16 FP32 stage launch: the pair form in the fast arithmetic (faster
 // than either column form at every size measured, 32^3 .. 512^3), else the
 // column form that shared_form() picks.
 template <bool FAST, int FORM>
 cudaError_t stage_column16(const StageArgs<float> &A, const LatticeParams<float> &P, const TileShape &shape,
                            const StageMaps &maps, int tma_ok, int *status, cudaStream_t s) {
-    if constexpr (FAST && dev::kPairForm<FORM>)
+    if constexpr (FAST)
         return stage_pair<FORM>(A, P, shape.pair_lz > 0 ? shape.pair_lz : shape.lz, maps, tma_ok, status, s);
     else if (shared_form(P, shape))
         return stage_column<float, FAST, FORM, 16, true>(A, P, shape.lz, maps, tma_ok, status, s);

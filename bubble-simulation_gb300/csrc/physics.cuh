@@ -399,15 +399,12 @@ BUBBLE_DEV R thermal_energy(R T, R phi, const LatticeParams<R> &P) {
     return P.a_rad * (t2 * t2) - (R(0.5) * P.th_g) * (t2 * (phi * phi));
 }
 // c_s^2 = (dp/dT) / (de/dT), held in [1e-4, 1] (an outer bound for HLL off the branch)
-template <typename R, bool FAST>
+template <typename R>
 BUBBLE_DEV R thermal_cs2(R T, R phi, const LatticeParams<R> &P) {
     const R t2 = T * T, f2 = phi * phi;
     const R dp = T * (R(4.0) * P.th_k * t2 - P.th_g * f2) + P.th_h * (f2 * phi);
     const R de = vmax(T * (R(4.0) * P.a_rad * t2 - P.th_g * f2), R(1e-30));
-    R c2;
-    if constexpr (FAST) c2 = dp * rcp_approx(de);
-    else c2 = dp / de;
-    return vmin(vmax(c2, R(1e-4)), R(1.0));
+    return vmin(vmax(dp / de, R(1e-4)), R(1.0));
 }
 // eos_temperature(p, phi): the root of p(T, phi) = p from the phi = 0 root,
 // each step held to [max(T_lo, T/2), 2T].
@@ -656,6 +653,7 @@ struct FaceSide {
 template <int AXIS, typename R, bool FAST, int FORM = kPlain>
 BUBBLE_DEV FaceSide<R> face_side(const V4<R> &q, R zmax2, const LatticeParams<R> &P, R phi = R(0)) {
     constexpr bool PERT = FORM == kPert;
+    static_assert(!FAST || FORM == kPlain || FORM == kMixed, "the other fast forms run in the pair form");
     FaceSide<R> s;
     R vx = q.x, vy = q.y, vz = q.z;
     const R p = q.w;
@@ -684,33 +682,20 @@ BUBBLE_DEV FaceSide<R> face_side(const V4<R> &q, R zmax2, const LatticeParams<R>
         if constexpr (FORM == kThermal) {
             const R T = thermal_temperature<R, FAST>(p, phi, P);
             enth = thermal_energy(T, phi, P) + p;
-            cs2 = thermal_cs2<R, FAST>(T, phi, P);
+            cs2 = thermal_cs2(T, phi, P);
         } else {
             enth = gamma_enthalpy(p, P);
             cs2 = P.eos_c2;
         }
-        R w, den_inv;
-        if constexpr (FAST) {
-            w = enth * rcp_approx(R(1.0) - v2);
-            den_inv = rcp_approx(R(1.0) - v2 * cs2);
-        } else {
-            w = enth / (R(1.0) - v2);
-        }
+        const R w = enth / (R(1.0) - v2);
         s.u = V4<R>{w - p, w * vx, w * vy, w * vz};
         const R cs = sqrt(cs2);
         const R rad = vmax((R(1.0) - v2) * (R(1.0) - vd * vd - cs2 * (v2 - vd * vd)), R(0.0));
-        if constexpr (FAST) {
-            const R a = vd * (R(1.0) - cs2) * den_inv;
-            const R b = cs * sqrt_approx(rad) * den_inv;
-            s.lm = a - b;
-            s.lp = a + b;
-        } else {
-            const R denom = R(1.0) - v2 * cs2;
-            const R a = vd * (R(1.0) - cs2) / denom;
-            const R b = cs * sqrt(rad) / denom;
-            s.lm = a - b;
-            s.lp = a + b;
-        }
+        const R denom = R(1.0) - v2 * cs2;
+        const R a = vd * (R(1.0) - cs2) / denom;
+        const R b = cs * sqrt(rad) / denom;
+        s.lm = a - b;
+        s.lp = a + b;
         s.f = V4<R>{(s.u.x + p) * vd, s.u.y * vd, s.u.z * vd, s.u.w * vd};
         if constexpr (AXIS == 0) s.f.y = s.f.y + p;
         if constexpr (AXIS == 1) s.f.z = s.f.z + p;
@@ -723,10 +708,10 @@ BUBBLE_DEV FaceSide<R> face_side(const V4<R> &q, R zmax2, const LatticeParams<R>
         // 1 - vd^2 - cs2 (v^2 - vd^2) = 1 - (2/3) vd^2 - v^2/3 for cs2 = 1/3;
         // E + p = w W^2, so the energy flux is w vd.
         const R om = R(1.0) - v2;
-        const R w = (R(4.0) * pf) * rcp_approx(om);
+        const R w = (R(4.0) * p) * rcp_approx(om);
         {
             const float2 uzw = p_mul(bc2(w), make_float2(vy, vz));
-            s.u = V4<R>{PERT ? __fmaf_rn(w, v2, __fmul_rn(R(3.0), p)) : w - p, w * vx, uzw.x, uzw.y};
+            s.u = V4<R>{w - p, w * vx, uzw.x, uzw.y};
         }
         const R inv_den = rcp_approx(__fmaf_rn(-v2, cs2, R(1.0)));
         const R tt = __fmaf_rn(-cs2, v2, __fmaf_rn(-(R(2.0) / R(3.0)), __fmul_rn(vd, vd), R(1.0)));

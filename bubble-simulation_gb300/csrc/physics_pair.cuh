@@ -1,7 +1,7 @@
 // Device-side physics of two lattice cells at once (fast arithmetic, FP32).
 //
-// The fast bag forms (plain, MIXED, perturbation) and the fast gamma law of
-// physics.cuh on pairs of cells: every quantity is a float2 whose halves belong to two different
+// The fast bag forms (plain, MIXED, perturbation), gamma law and thermal
+// potential of physics.cuh on pairs of cells: every quantity is a float2 whose halves belong to two different
 // cells, so the paired FP32 instructions of sm_100+ (two IEEE operations per
 // issue slot) carry the whole solver, with no exchange between the halves.
 // The formulas are those of the shaders cited in physics.cuh; every rounding
@@ -63,6 +63,68 @@ BUBBLE_DEV void face_states_pair(const P4 &qm, const P4 &q, const P4 &qp, float 
 }
 
 // ---------------------------------------------------------------------------
+//  Thermal potential: temperature of two cells
+// ---------------------------------------------------------------------------
+// thermal_temperature of one cell: eight bounded steps.  Out of line: only
+// where the short iteration below did not converge.
+static __device__ __noinline__ float temperature_slow(float p, float phi, float th_k, float th_g, float th_h, float th_lo,
+                                               float p_floor) {
+    LatticeParams<float> P{};
+    P.th_k = th_k;
+    P.th_g = th_g;
+    P.th_h = th_h;
+    P.th_lo = th_lo;
+    P.p_floor = p_floor;
+    return thermal_temperature<float, true>(p, phi, P);
+}
+
+// The phi-dependent constants of p(T) = k T^4 - b T^2 + h T (b = gamma phi^2 / 2, h = A phi^3 / 3).
+struct ThermalPair {
+    float2 phi, b, h;
+};
+BUBBLE_DEV ThermalPair thermal_pair(float2 phi, const LatticeParams<float> &P) {
+    const float2 f2 = p_mul(phi, phi);
+    return ThermalPair{phi, p_mul(bc2(0.5f * P.th_g), f2), p_mul(bc2(P.th_h), p_mul(f2, phi))};
+}
+// dp/dT = T (4k T^2 - 2b) + h
+BUBBLE_DEV float2 thermal_dp(float2 t, float2 t2, const ThermalPair &f, const LatticeParams<float> &P) {
+    return p_fma(t, p_fma(bc2(4.0f * P.th_k), t2, p_mul(bc2(-2.0f), f.b)), f.h);
+}
+// One Newton step of p(T) = p; returns the step.
+BUBBLE_DEV float2 thermal_step(float2 &t, float2 p, const ThermalPair &f, const LatticeParams<float> &P) {
+    const float2 t2 = p_mul(t, t);
+    const float2 g = p_fma(p_fma(bc2(P.th_k), t2, p_mul(bc2(-1.0f), f.b)), t2, p_sub(p_mul(f.h, t), p));
+    const float2 d = p_mul(g, rcp2(thermal_dp(t, t2, f, P)));
+    t = p_sub(t, d);
+    return d;
+}
+// eos_temperature(p, phi).  Newton's steps converge quadratically from the phi
+// = 0 root: where the first is below 1e-4 T its successor is below rounding
+// (all of the symmetric phase); otherwise three more follow, and a cell whose
+// last step is still above 2e-4 T, or that left the branch T >= lo |phi|, takes
+// the bounded iteration.  Values accepted early are within 7.4e-8 T of the
+// root (64-bit evaluation over T >= 0.4 T_ref, -0.3 <= phi/phi_b <= 1.2 and the
+// validated gamma and A).  Each half is decided on its own values, so a pair's
+// halves do not affect each other.
+BUBBLE_DEV float2 temperature_pair(float2 p, const ThermalPair &f, const LatticeParams<float> &P) {
+    const float2 t0 = sqrt2(sqrt2(p_mul(p, bc2(P.th_ik))));
+    float2 t1 = t0;
+    const float2 d1 = thermal_step(t1, p, f, P);
+    const bool cx = fabsf(d1.x) <= 1e-4f * t1.x, cy = fabsf(d1.y) <= 1e-4f * t1.y;
+    if (cx && cy) return t1;
+    float2 t = t1;
+    thermal_step(t, p, f, P);
+    thermal_step(t, p, f, P);
+    const float2 d = thermal_step(t, p, f, P);
+    const float lx = P.th_lo * fabsf(f.phi.x), ly = P.th_lo * fabsf(f.phi.y);
+    if (!cx && !(fabsf(d.x) <= 2e-4f * t.x && t.x >= lx))
+        t.x = temperature_slow(p.x, f.phi.x, P.th_k, P.th_g, P.th_h, P.th_lo, P.p_floor);
+    if (!cy && !(fabsf(d.y) <= 2e-4f * t.y && t.y >= ly))
+        t.y = temperature_slow(p.y, f.phi.y, P.th_k, P.th_g, P.th_h, P.th_lo, P.p_floor);
+    return make_float2(cx ? t1.x : t.x, cy ? t1.y : t.y);
+}
+
+// ---------------------------------------------------------------------------
 //  Primitive recovery
 // ---------------------------------------------------------------------------
 // One cell through the scalar recovery (|Z| cap, FP64 above gamma = 3,
@@ -85,6 +147,22 @@ __device__ __noinline__ V4<float> recover_slow(V4<float> u, float e_floor, float
     return recover_sanitised<float, true, FORM>(u, P, 0.0f, z_max * z_max);
 }
 
+// The same for the thermal potential, whose recovery depends on phi.
+static __device__ __noinline__ V4<float> recover_slow_thermal(V4<float> u, float phi, float e_floor, float z_max,
+                                                       float p_floor, float th_k, float th_g, float th_h,
+                                                       float th_i2a, float a_rad) {
+    LatticeParams<float> P{};
+    P.e_floor = e_floor;
+    P.z_max = z_max;
+    P.p_floor = p_floor;
+    P.th_k = th_k;
+    P.th_g = th_g;
+    P.th_h = th_h;
+    P.th_i2a = th_i2a;
+    P.a_rad = a_rad;
+    return recover_sanitised<float, true, kThermal>(u, P, phi, z_max * z_max);
+}
+
 // sanitise(recover(u)) of two cells in two parts, so independent work can be
 // scheduled between them: recover_pair evaluates both cells by the formulas
 // that hold below gamma = 3; recover_fix sends a cell whose |v|^2 came out
@@ -92,7 +170,7 @@ __device__ __noinline__ V4<float> recover_slow(V4<float> u, float e_floor, float
 // whose |Z| exceeds z_max E: the cap leaves |v|^2 > 8/9, and without it the
 // result is larger still (p is floored when E^2 - Z^2 is not positive).
 template <int FORM>
-BUBBLE_DEV P4 recover_pair(const V4<float> &ua, const V4<float> &ub, const LatticeParams<float> &P) {
+BUBBLE_DEV P4 recover_pair(const V4<float> &ua, const V4<float> &ub, float2 phi, const LatticeParams<float> &P) {
     const float2 de = max2(make_float2(ua.x, ub.x), P.e_floor);
     const float2 zx = make_float2(ua.y, ub.y), zy = make_float2(ua.z, ub.z), zz = make_float2(ua.w, ub.w);
     const float2 z2 = dot3_2(zx, zy, zz);
@@ -109,6 +187,40 @@ BUBBLE_DEV P4 recover_pair(const V4<float> &ua, const V4<float> &ub, const Latti
         const float2 inv = rcp2(p_add(de, p));
         return P4{p_mul(zx, inv), p_mul(zy, inv), p_mul(zz, inv), p};
     }
+    if constexpr (FORM == kThermal) {
+        // Newton on f(p) = p - p(T(e), phi) from the Z = 0 root, e = E - Z^2 / (E
+        // + p): three steps; a cell whose last step is above 2e-4 p gets v out
+        // of range, which sends it to recover_fix
+        const ThermalPair f = thermal_pair(phi, P);
+        const float2 a4 = bc2(4.0f * P.a_rad), b2 = p_mul(f.b, f.b);
+        float2 p, dp = make_float2(0.0f, 0.0f), e = de, isp = dp;
+#pragma unroll
+        for (int it = 0; it <= 3; ++it) {
+            if (it > 0) {
+                isp = rcp2(p_add(de, p));
+                e = p_sub(de, p_mul(z2, isp));
+            }
+            const float2 x = p_mul(p_add(f.b, sqrt2(p_fma(a4, e, b2))), bc2(P.th_i2a));
+            const float2 t = sqrt2(x);
+            const float2 pt = p_fma(p_sub(p_mul(bc2(P.th_k), x), f.b), x, p_mul(f.h, t));  // p(T(e), phi)
+            if (it == 0) {
+                p = max2(pt, P.p_floor);
+            } else {
+                const float2 dpt = thermal_dp(t, x, f, P);
+                const float2 det = max2(p_mul(t, p_fma(a4, x, p_mul(bc2(-2.0f), f.b))), 1e-30f);
+                float2 c2 = p_mul(dpt, rcp2(det));
+                c2 = make_float2(fminf(fmaxf(c2.x, 1e-4f), 1.0f), fminf(fmaxf(c2.y, 1e-4f), 1.0f));
+                const float2 d = p_fma(p_mul(c2, p_mul(z2, bc2(-1.0f))), p_mul(isp, isp), bc2(1.0f));
+                dp = p_mul(p_sub(p, pt), rcp2(d));
+                p = max2(p_sub(p, dp), P.p_floor);
+            }
+        }
+        const float2 inv = rcp2(p_add(de, p));
+        P4 q{p_mul(zx, inv), p_mul(zy, inv), p_mul(zz, inv), p};
+        if (!(fabsf(dp.x) <= 2e-4f * p.x)) q.x.x = 2.0f;
+        if (!(fabsf(dp.y) <= 2e-4f * p.y)) q.x.y = 2.0f;
+        return q;
+    }
     const float2 e = FORM == kPert ? p_add(bc2(P.e_bg), de) : de;
     const float2 sq = sqrt2(p_fma(p_mul(bc2(4.0f), e), e, p_mul(bc2(-3.0f), z2)));
     float2 p, s;
@@ -124,20 +236,28 @@ BUBBLE_DEV P4 recover_pair(const V4<float> &ua, const V4<float> &ub, const Latti
     return P4{p_mul(zx, inv), p_mul(zy, inv), p_mul(zz, inv), p};
 }
 template <int FORM>
-BUBBLE_DEV void recover_fix(P4 &q, const V4<float> *ua, const V4<float> *ub, const LatticeParams<float> &P) {
+BUBBLE_DEV void recover_fix(P4 &q, const V4<float> *ua, const V4<float> *ub, float2 phi,
+                            const LatticeParams<float> &P) {
     const float2 v2 = dot3_2(q.x, q.y, q.z);
     constexpr float kFast = 8.0f / 9.0f;
     if (fmaxf(v2.x, v2.y) > kFast) {
-        const float c0 = FORM == kGamma ? P.eos_c2 : P.e_bg, c1 = FORM == kGamma ? P.eos_e0 : P.p_bg;
+        auto slow = [&](const V4<float> *u, float f) {
+            if constexpr (FORM == kThermal)
+                return recover_slow_thermal(*u, f, P.e_floor, P.z_max, P.p_floor, P.th_k, P.th_g, P.th_h, P.th_i2a,
+                                            P.a_rad);
+            else
+                return recover_slow<FORM>(*u, P.e_floor, P.z_max, P.p_floor, FORM == kGamma ? P.eos_c2 : P.e_bg,
+                                          FORM == kGamma ? P.eos_e0 : P.p_bg);
+        };
         if (v2.x > kFast) {
-            const V4<float> r = recover_slow<FORM>(*ua, P.e_floor, P.z_max, P.p_floor, c0, c1);
+            const V4<float> r = slow(ua, phi.x);
             q.x.x = r.x;
             q.y.x = r.y;
             q.z.x = r.z;
             q.w.x = r.w;
         }
         if (v2.y > kFast) {
-            const V4<float> r = recover_slow<FORM>(*ub, P.e_floor, P.z_max, P.p_floor, c0, c1);
+            const V4<float> r = slow(ub, phi.y);
             q.x.y = r.x;
             q.y.y = r.y;
             q.z.y = r.z;
@@ -158,18 +278,34 @@ struct PairSide {
 // (2 vd -+ sqrt((1 - v^2) T)) / D are those of face_side: numerator and
 // denominator scaled by 3.
 template <int AXIS, int FORM>
-BUBBLE_DEV PairSide pair_side(const P4 &q, float2 v2, const LatticeParams<float> &P) {
+BUBBLE_DEV PairSide pair_side(const P4 &q, float2 v2, float2 phi, const LatticeParams<float> &P) {
     PairSide s;
     const float2 vd = AXIS == 0 ? q.x : (AXIS == 1 ? q.y : q.z);
     const float2 p = q.w;
     const float2 om = p_sub(bc2(1.0f), v2);
     const float2 pf = FORM == kPert ? p_add(bc2(P.p_bg), p) : p;  // the full pressure
-    const float2 w = p_mul(FORM == kGamma ? p_fma(bc2(P.eos_k), p, bc2(P.eos_e0)) : p_mul(bc2(4.0f), pf), rcp2(om));
+    float2 cs2 = om, enth = om;  // thermal: c_s^2 and the enthalpy density at T(p, phi)
+    if constexpr (FORM == kThermal) {
+        const ThermalPair f = thermal_pair(phi, P);
+        const float2 t = temperature_pair(p, f, P), t2 = p_mul(t, t);
+        enth = p_fma(p_sub(p_mul(bc2(P.a_rad), t2), f.b), t2, p);
+        const float2 de = max2(p_mul(t, p_fma(bc2(4.0f * P.a_rad), t2, p_mul(bc2(-2.0f), f.b))), 1e-30f);
+        cs2 = p_mul(thermal_dp(t, t2, f, P), rcp2(de));
+        cs2 = make_float2(fminf(fmaxf(cs2.x, 1e-4f), 1.0f), fminf(fmaxf(cs2.y, 1e-4f), 1.0f));
+    }
+    const float2 w = p_mul(FORM == kThermal ? enth : FORM == kGamma ? p_fma(bc2(P.eos_k), p, bc2(P.eos_e0)) : p_mul(bc2(4.0f), pf), rcp2(om));
     s.u.x = FORM == kPert ? p_fma(w, v2, p_mul(bc2(3.0f), p)) : p_sub(w, p);
     s.u.y = p_mul(w, q.x);
     s.u.z = p_mul(w, q.y);
     s.u.w = p_mul(w, q.z);
-    if constexpr (FORM == kGamma) {
+    if constexpr (FORM == kThermal) {
+        const float2 d = p_fma(v2, p_mul(cs2, bc2(-1.0f)), bc2(1.0f));
+        const float2 inv = rcp2(d);
+        const float2 tv = p_mul(vd, p_sub(cs2, bc2(1.0f)));
+        const float2 sq = sqrt2(p_mul(cs2, p_mul(om, p_fma(tv, vd, d))));
+        s.nlm = p_mul(p_add(sq, tv), inv);
+        s.lp = p_mul(p_sub(sq, tv), inv);
+    } else if constexpr (FORM == kGamma) {
         // the same with c_s^2 = c2, unscaled: D = 1 - c2 v^2, T = D - (1 - c2) vd^2
         const float2 d = p_fma(v2, bc2(-P.eos_c2), bc2(1.0f));
         const float2 inv = rcp2(d);
@@ -213,12 +349,13 @@ BUBBLE_DEV void clamp_pair(P4 &q, float2 &v2, float zmax2, bool exchanged) {
 // One side of a face pair and its |v|^2.  `exchanged`: q holds (vy, vx, vz,
 // p), for a y face taken as AXIS 0; the flux is then (E, Zy, Zx, Zz) with the
 // bits of AXIS 1.
+// fl, fr: the field in the two sides' own cells, read by the thermal form only.
 struct FacePair {
     P4 l, r;
-    float2 vl, vr;
+    float2 vl, vr, fl, fr;
 };
-BUBBLE_DEV FacePair face_pair(const P4 &l, const P4 &r, bool exchanged = false) {
-    return FacePair{l, r, speed2(l, exchanged), speed2(r, exchanged)};
+BUBBLE_DEV FacePair face_pair(const P4 &l, const P4 &r, float2 fl, float2 fr, bool exchanged = false) {
+    return FacePair{l, r, speed2(l, exchanged), speed2(r, exchanged), fl, fr};
 }
 BUBBLE_DEV float max_speed2(const FacePair &f) {
     return fmaxf(fmaxf(f.vl.x, f.vl.y), fmaxf(f.vr.x, f.vr.y));
@@ -231,8 +368,8 @@ BUBBLE_DEV void clamp_face(FacePair &f, float zmax2, bool exchanged = false) {
 
 template <int AXIS, int FORM>
 BUBBLE_DEV P4 hll_pair(const FacePair &f, const LatticeParams<float> &P) {
-    const PairSide L = pair_side<AXIS, FORM>(f.l, f.vl, P);
-    const PairSide R = pair_side<AXIS, FORM>(f.r, f.vr, P);
+    const PairSide L = pair_side<AXIS, FORM>(f.l, f.vl, f.fl, P);
+    const PairSide R = pair_side<AXIS, FORM>(f.r, f.vr, f.fr, P);
     const float2 ns = make_float2(fmaxf(fmaxf(L.nlm.x, R.nlm.x), 0.0f), fmaxf(fmaxf(L.nlm.y, R.nlm.y), 0.0f));
     const float2 sx = make_float2(fmaxf(fmaxf(L.lp.x, R.lp.x), 0.0f), fmaxf(fmaxf(L.lp.y, R.lp.y), 0.0f));
     // (s_max f_L - s_min f_R + s_min s_max (u_R - u_L)) / (s_max - s_min)

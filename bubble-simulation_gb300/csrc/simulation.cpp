@@ -283,6 +283,7 @@ LatticeParams<float> lattice_params_f32(const bubble_spec &spec) {
         p.th_a = a;
         p.th_lo = std::sqrt(3.0f * g / (4.0f * h.a_rad));
         p.th_i2a = 1.0f / (2.0f * h.a_rad);
+        p.th_ik = (float)(1.0 / (double)p.th_k);
         p.a_rad = h.a_rad;
         p.t_ref = h.t_ref;
     }

@@ -15,8 +15,8 @@
 //   * two halo warps recover the cross-shaped halo ring of each plane and
 //     compute the face states and fluxes on the tile's far edges.
 //
-// Runs the strict arithmetic, FP64, the thermal form and the 32-wide tiles;
-// the other fast forms on 16 x 16 tiles run in the pair form (stage_pair.cuh).
+// Runs the strict arithmetic, FP64 and the 32-wide tiles; the fast arithmetic
+// on 16 x 16 tiles runs in the pair form (stage_pair.cuh).
 //
 // Two forms of the same arithmetic (template flag LEAN):
 //   * register form: the column's z pipeline (the primitives and phi of the

@@ -1,5 +1,5 @@
-// Fused SSP-RK3 stage kernel, pair form: the fast FP32 bag forms (plain,
-// MIXED, perturbation) and the fast gamma law on 16 x 16 tiles.
+// Fused SSP-RK3 stage kernel, pair form: the fast arithmetic (FP32, every
+// form and equation of state) on 16 x 16 tiles.
 //
 // The scheme of stage_column.cuh (z-marching column tile, three phases and
 // two barriers per plane, TMA-staged raw planes) with two cells per thread:
@@ -29,7 +29,9 @@
 // unrolled by 2 or 3 (20 to 30 % slower).  Step time, column form to pair
 // form (GB300): 512^3 MIXED 10.85 -> 8.18 ms, 256^3 perturbation 1.54 -> 1.16
 // ms, 128^3 0.212 -> 0.170 ms, 64^3 49.3 -> 43.1 us; the gamma law at 128^3,
-// with its recovery in closed form, 0.33 -> 0.18 ms.
+// with its recovery in closed form, 0.33 -> 0.18 ms, the thermal potential at
+// 96^3, with its short iterations, 0.374 -> 0.177 ms (0.240 at two CTAs per SM,
+// where it has no spills).
 //
 // Every tile is processed in full: a tile that reaches past the lattice
 // stages the wrapped cells beyond the edge, so the faces and neighbours of
@@ -50,10 +52,6 @@
 
 namespace bubble {
 namespace dev {
-
-// The forms that run as pairs in the fast arithmetic on 16 x 16 tiles.
-template <int FORM>
-constexpr bool kPairForm = FORM == kPlain || FORM == kMixed || FORM == kPert || FORM == kGamma;
 
 struct PairLayout {
     static constexpr int TX = 16, TY = 16;
@@ -282,16 +280,25 @@ BUBBLE_DEV bool pair_item(unsigned char *smem, const StageArgs<float> &A, const 
             const uint32_t pa = (uint32_t)wrap1(z0 - 2, P.nz) * plane, pb = (uint32_t)wrap1(z0 - 1, P.nz) * plane;
             const V4<float> a0 = A.fluid_in[pa + g0], a1 = A.fluid_in[pa + g1];
             const V4<float> b0 = A.fluid_in[pb + g0], b1 = A.fluid_in[pb + g1];
-            q0 = recover_pair<FORM>(a0, a1, P);
-            recover_fix<FORM>(q0, &a0, &a1, P);
-            q1 = recover_pair<FORM>(b0, b1, P);
-            recover_fix<FORM>(q1, &b0, &b1, P);
-            phi_slot(z0 - 1)[pc] = make_float2(A.field_in[pb + g0].x, A.field_in[pb + g1].x);
+            const float2 fa = make_float2(A.field_in[pa + g0].x, A.field_in[pa + g1].x);
+            const float2 fb = make_float2(A.field_in[pb + g0].x, A.field_in[pb + g1].x);
+            q0 = recover_pair<FORM>(a0, a1, fa, P);
+            recover_fix<FORM>(q0, &a0, &a1, fa, P);
+            q1 = recover_pair<FORM>(b0, b1, fb, P);
+            recover_fix<FORM>(q1, &b0, &b1, fb, P);
+            phi_slot(z0 - 2)[pc] = fa;
+            phi_slot(z0 - 1)[pc] = fb;
         }
         const int ix = cj * FXW + ci, iy = cj * 16 + ci;
         const bool v0 = ci < xe && cj < ye, v1 = ci < xe && cj + 8 < ye;
         if (!wait_raw(z0, true)) *dead = 1;
         plane_barrier();
+
+        // phi of plane p beside the thread's pair, for the thermal form's faces
+        auto phi_at = [&](int p, int d) {
+            if constexpr (FORM == kThermal) return phi_slot(p)[pc + d];
+            else return zero;
+        };
 
         // One plane; the planes below z0 (ACT false) only fill the z pipeline.
         auto march = [&](int z, auto act) {
@@ -301,13 +308,11 @@ BUBBLE_DEV bool pair_item(unsigned char *smem, const StageArgs<float> &A, const 
             const V2<float> *rf = raw_f + raw_slot(z + 2) * PC + rc;
             float2 *wf = phi_slot(z + 2) + pc;
             P4 lox, loy;
-            P4 q2 = recover_pair<FORM>(ru[0], ru[8 * PW], P);
-            {
-                const float2 f = make_float2(rf[0].x, rf[8 * PW].x);
-                wf[0] = f;
-                if (cj == 0) wf[8 * PQ].x = f.y;   // row 8 in pair row 8
-                if (cj == 7) wf[-8 * PQ].y = f.x;  // row 7 in pair row -1
-            }
+            const float2 f2 = make_float2(rf[0].x, rf[8 * PW].x);
+            P4 q2 = recover_pair<FORM>(ru[0], ru[8 * PW], f2, P);
+            wf[0] = f2;
+            if (cj == 0) wf[8 * PQ].x = f2.y;   // row 8 in pair row 8
+            if (cj == 7) wf[-8 * PQ].y = f2.x;  // row 7 in pair row -1
             if constexpr (ACT) {
                 P4 up;
                 face_states_pair(get_pair<PP>(pr, pc - 1), q0, get_pair<PP>(pr, pc + 1), P.p_floor, lox, up);
@@ -317,12 +322,12 @@ BUBBLE_DEV bool pair_item(unsigned char *smem, const StageArgs<float> &A, const 
                 // the upper y state of row 7 is the lower side of face 8: second half of face pair 0
                 if (cj == 7) put_half<FY, 0, 1>(hy, ci, up);
             }
-            recover_fix<FORM>(q2, ru, ru + 8 * PW, P);
+            recover_fix<FORM>(q2, ru, ru + 8 * PW, f2, P);
             P4 fz_p;
             {
                 P4 lo, up;
                 face_states_pair(q0, q1, q2, P.p_floor, lo, up);
-                FacePair f = face_pair(hiz, lo);
+                FacePair f = face_pair(hiz, lo, phi_at(z, 0), phi_at(z + 1, 0));
                 if (max_speed2(f) > zmax2) clamp_face(f, zmax2);
                 fz_p = hll_pair<2, FORM>(f, P);
                 hiz = up;
@@ -338,7 +343,7 @@ BUBBLE_DEV bool pair_item(unsigned char *smem, const StageArgs<float> &A, const 
             P4 yl;
             const uint32_t base = (uint32_t)z * plane;
             if constexpr (ACT) {
-                FacePair f = face_pair(get_pair<FX>(hx, ix), lox);
+                FacePair f = face_pair(get_pair<FX>(hx, ix), lox, phi_at(z, -1), phi_at(z, 0));
                 if (max_speed2(f) > zmax2) clamp_face(f, zmax2);
                 put_pair<FX>(fx, ix, hll_pair<0, FORM>(f, P));
                 // cells beyond the edge load their wrapped images and are not stored
@@ -352,7 +357,7 @@ BUBBLE_DEV bool pair_item(unsigned char *smem, const StageArgs<float> &A, const 
                     un0 = A.fluid_n[base + g0];
                     un1 = A.fluid_n[base + g1];
                 }
-                f = face_pair(get_pair<FY>(hy, iy), loy);
+                f = face_pair(get_pair<FY>(hy, iy), loy, phi_at(z, -PQ), phi_at(z, 0));
                 if (max_speed2(f) > zmax2) clamp_face(f, zmax2);
                 yl = hll_pair<1, FORM>(f, P);
                 put_pair<FY>(fy, iy, yl);
@@ -379,7 +384,16 @@ BUBBLE_DEV bool pair_item(unsigned char *smem, const StageArgs<float> &A, const 
                 const float2 gam = make_float2(rsqrt_approx(fmaxf(om.x, 1e-12f)), rsqrt_approx(fmaxf(om.y, 1e-12f)));
                 const float2 vg = p_fma(q0.z, gz, p_fma(q0.y, gy, p_mul(q0.x, gx)));
                 const float2 drag = p_mul(bc2(P.eta), p_mul(gam, p_add(pi, vg)));
-                const float2 dpot = p_mul(phi, p_fma(p_fma(bc2(P.lambda), phi, bc2(-P.delta)), phi, bc2(P.m2)));
+                float2 dpot = p_mul(phi, p_fma(p_fma(bc2(P.lambda), phi, bc2(-P.delta)), phi, bc2(P.m2)));
+                float2 src = drag;
+                if constexpr (FORM == kThermal) {
+                    // the thermal part of dV/dphi, and its plasma part, exchanged like the friction
+                    const float2 t = temperature_pair(q0.w, thermal_pair(phi, P), P);
+                    const float2 dt = p_sub(t, bc2(P.t_ref));
+                    const float2 gt = p_mul(bc2(P.th_g), p_mul(dt, p_add(t, bc2(P.t_ref))));
+                    dpot = p_fma(phi, p_fma(p_mul(bc2(-P.th_a), dt), phi, gt), dpot);
+                    src = p_fma(phi, p_fma(p_mul(bc2(-P.th_a), t), phi, p_mul(bc2(P.th_g), p_mul(t, t))), drag);
+                }
                 const float2 d_pi = p_sub(p_sub(lap, dpot), drag);
                 // minus the flux divergence: ((dx + dy) + dz) / dx
                 const P4 xl = get_pair<FX>(fx, ix), xu = get_pair<FX>(fx, ix + 1);
@@ -387,8 +401,8 @@ BUBBLE_DEV bool pair_item(unsigned char *smem, const StageArgs<float> &A, const 
                 auto div = [&](float2 a, float2 b, float2 c, float2 d, float2 e, float2 f) {
                     return p_mul(p_add(p_add(p_sub(a, b), p_sub(c, d)), p_sub(e, f)), inv_dx);
                 };
-                const float2 nd = p_mul(drag, bc2(-1.0f));
-                const float2 d_e = p_fma(drag, pi, div(xl.x, xu.x, yl.x, yu.x, fz_m.x, fz_p.x));
+                const float2 nd = p_mul(src, bc2(-1.0f));
+                const float2 d_e = p_fma(src, pi, div(xl.x, xu.x, yl.x, yu.x, fz_m.x, fz_p.x));
                 const float2 d_x = p_fma(nd, gx, div(xl.y, xu.y, yl.y, yu.y, fz_m.y, fz_p.y));
                 const float2 d_y = p_fma(nd, gy, div(xl.z, xu.z, yl.z, yu.z, fz_m.z, fz_p.z));
                 const float2 d_z = p_fma(nd, gz, div(xl.w, xu.w, yl.w, yu.w, fz_m.w, fz_p.w));
@@ -421,11 +435,12 @@ BUBBLE_DEV bool pair_item(unsigned char *smem, const StageArgs<float> &A, const 
             const V4<float> *ru = raw_u + raw_slot(z + 2) * PC;
             const V2<float> *rf = raw_f + raw_slot(z + 2) * PC;
             float2 *wf = phi_slot(z + 2);
-            P4 q2 = recover_pair<FORM>(ru[rc], ru[rc + 8 * PW], P);
-            P4 s2 = recover_pair<FORM>(ru[r1a], ru[r1b], P);
-            wf[pc] = make_float2(rf[rc].x, rf[rc + 8 * PW].x);
-            wf[p1a].x = rf[r1a].x;
-            wf[p1b].y = rf[r1b].x;
+            const float2 f2 = make_float2(rf[rc].x, rf[rc + 8 * PW].x), f3 = make_float2(rf[r1a].x, rf[r1b].x);
+            P4 q2 = recover_pair<FORM>(ru[rc], ru[rc + 8 * PW], f2, P);
+            P4 s2 = recover_pair<FORM>(ru[r1a], ru[r1b], f3, P);
+            wf[pc] = f2;
+            wf[p1a].x = f3.x;
+            wf[p1b].y = f3.y;
             if (act) {
                 P4 a, b, c, lo, up;
                 if (xs) {
@@ -454,8 +469,8 @@ BUBBLE_DEV bool pair_item(unsigned char *smem, const StageArgs<float> &A, const 
                     ly[h & 15] = make_float4(lo.x.y, lo.y.y, lo.z.y, lo.w.y);
                 }
             }
-            recover_fix<FORM>(q2, ru + rc, ru + rc + 8 * PW, P);
-            recover_fix<FORM>(s2, ru + r1a, ru + r1b, P);
+            recover_fix<FORM>(q2, ru + rc, ru + rc + 8 * PW, f2, P);
+            recover_fix<FORM>(s2, ru + r1a, ru + r1b, f3, P);
             plane_barrier();
             if (z + 4 <= zlast) issue(z + 4);
             if (A.stage != 0 && z + kAhead >= z0 && z + kAhead < z1 && (h & 15) < ye) {
@@ -486,7 +501,18 @@ BUBBLE_DEV bool pair_item(unsigned char *smem, const StageArgs<float> &A, const 
                     const float4 c = ly[i], d = ly[h];
                     r = P4{make_float2(c.y, d.y), make_float2(c.x, d.x), make_float2(c.z, d.z), make_float2(c.w, d.w)};
                 }
-                FacePair f = face_pair(l, r, !xf);
+                float2 pl{}, pq{};
+                if constexpr (FORM == kThermal) {
+                    const float2 *fz = phi_slot(z);
+                    if (xf) {  // columns 15 and 16
+                        pl = fz[(h + 2) * PQ + 17];
+                        pq = fz[(h + 2) * PQ + 18];
+                    } else {  // rows 15 and 16 of the two columns
+                        pl = make_float2(fz[9 * PQ + i + 2].y, fz[9 * PQ + h + 2].y);
+                        pq = make_float2(fz[10 * PQ + i + 2].y, fz[10 * PQ + h + 2].y);
+                    }
+                }
+                FacePair f = face_pair(l, r, pl, pq, !xf);
                 if (max_speed2(f) > zmax2) clamp_face(f, zmax2, !xf);
                 P4 fl = hll_pair<0, FORM>(f, P);
                 if (xf) {

@@ -26,16 +26,14 @@ int bubble_ext_set_path(bubble_sim *sim, int32_t path);
  * for 16 x 16 tiles, the default, in every form; 8 for 32 x 8 in the plain
  * and MIXED forms; 4 for 32 x 4 in those forms with the fast arithmetic;
  * FP64: 16 (default) or 4 for 32 x 4) and z chunk (planes marched per CTA).
- * Until it is set, those fast forms of 16 x 16 tiles that run two cells per
- * thread (see bubble_ext_set_stage_form) pick a chunk of their own and the chunk
+ * Until it is set, the fast arithmetic picks a chunk of its own and the chunk
  * reported is the column kernel's. */
 int bubble_ext_set_tile(bubble_sim *sim, int32_t ty, int32_t lz);
 int bubble_ext_get_tile(const bubble_sim *sim, int32_t *ty, int32_t *lz);
 
 /* Form of the fused column kernel for FP32 16 x 16 tiles; both forms give
- * identical bits.  The fast arithmetic of the bag equation of state (SINGLE,
- * MIXED, PERTURBATION) and of the gamma law has one form of its own, two
- * cells per thread, and runs it whatever is set here.  REGISTERS keeps each column's z pipeline in registers
+ * identical bits.  The fast arithmetic has one form of its own, two cells per
+ * thread, and runs it whatever is set here.  REGISTERS keeps each column's z pipeline in registers
  * (two CTAs per SM); SHARED reads it back from shared memory (three CTAs
  * per SM, faster once a launch fills more than one wave); AUTO (default)
  * takes the form a cost model of the launch rates cheaper for the lattice

@@ -74,14 +74,20 @@ def test_pair_form(bubble, oracle_mod, gpu, grid, precision):
         assert np.array_equal(got[0], fast[0]) and np.array_equal(got[1], fast[1]), lz
 
 
-@pytest.mark.parametrize("eos_param", [(1.2, 0.05), (2.0, 0.0), (1.02, 0.12)])
+E_REF = 0.125  # e_ref = a_rad of the default model
+EOS = [("gamma_law", (1.2, 0.05)), ("gamma_law", (2.0, 0.0)), ("gamma_law", (1.02, 0.12)), ("thermal", (0.0, 0.0)),
+       ("thermal", (0.0125, 0.05)), ("thermal", (0.999 * E_REF / 6.0, 0.999 * E_REF / np.sqrt(2.0)))]
+
+
+@pytest.mark.parametrize("eos,eos_param", EOS)
 @pytest.mark.parametrize("grid", GRIDS)
-def test_pair_form_gamma_law(bubble, oracle_mod, gpu, grid, eos_param):
-    """The gamma law's pair form (closed-form recovery) against the strict form
-    (eight Newton steps): the fast arithmetic's bar of 1e-5 per component, and
-    the same bits for every chunking."""
+def test_pair_form_other_equations_of_state(bubble, oracle_mod, gpu, grid, eos, eos_param):
+    """The gamma law's closed-form recovery and the thermal potential's short
+    iterations against the strict form's eight Newton steps: the fast
+    arithmetic's bar of 1e-5 per component, and the same bits for every
+    chunking."""
     f0, u0, _ = _state(oracle_mod, grid, "single")
-    kw = dict(eos="gamma_law", eos_param=eos_param)
+    kw = dict(eos=eos, eos_param=eos_param)
     strict = _run(bubble, grid, f0, u0, "single", "strict", **kw)
     fast = _run(bubble, grid, f0, u0, "single", "fast", **kw)
     for a, s in zip(fast, strict):
