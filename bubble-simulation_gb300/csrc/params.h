@@ -113,6 +113,23 @@ inline double column_stage_cost(uint32_t nx, uint32_t ny, uint32_t nz, int lz, b
     return ((double)(rounds - 1) * p + p_last) * (double)(lz_eff + 2);
 }
 
+// Cost model of one FP64 stage launch, in plane times of a CTA.  The FP64 pipes
+// bound it (two operations per clock and SM on GB300), so an SM's time is the
+// sum of its CTAs' planes, each chunk costing 0.73 of a plane for its warm-up:
+// 16 x 16 tiles measure 238 us (lz + 0.73) per step over lz = 2 .. 64 where
+// every CTA has an SM.  The shorter last chunks fill the SMs that the full
+// ones leave free.
+inline double fp64_stage_cost(long tiles, int nz, int lz, int sms) {
+    if (lz < 1) lz = 1;
+    if (sms < 1) sms = 1;
+    const double a = lz + 0.73, b = nz % lz + 0.73;  // a full chunk, the last one
+    const long full = tiles * (nz / lz), rest = nz % lz ? tiles : 0;
+    const long m = full / sms, x = full % sms;  // every SM has m full chunks, x of them one more
+    const double cost = (double)(x ? m + 1 : m) * a;
+    const long room = x ? (sms - x) * (long)(a / b) : 0;
+    return rest <= room ? cost : cost + (double)((rest - room + sms - 1) / sms) * b;
+}
+
 // Cost model of one stage launch in the pair form, in plane times of a CTA
 // that shares its SM with two others (2.5 us on GB300).  Three CTAs fit on an
 // SM; a plane takes 0.57 with one there, 0.77 with two.  A chunk costs its

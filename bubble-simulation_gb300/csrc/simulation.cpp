@@ -75,7 +75,22 @@ int default_chunk(const uint32_t grid[3], int ty, bool fp32) {
     }
     const long tx = tile_x_for(ty);
     const long tiles = (long)((grid[0] + tx - 1) / tx) * (long)((grid[1] + ty - 1) / ty);
-    // Other tiles and FP64, two regimes (measured with 32 x 8 tiles, ms per
+    if (!fp32) {
+        // the cheapest chunk of the FP64 model, ties to longer ones (us per step,
+        // chunks of 8 planes or more and the pick: 32^3 2081 and 412, 64^3 2081
+        // and 1843, 96^3 6067 and 5655)
+        double best = 1e300;
+        int best_lz = (int)grid[2];
+        for (int lz = (int)grid[2]; lz >= 1; --lz) {
+            const double c = fp64_stage_cost(tiles, (int)grid[2], lz, sms);
+            if (c < best * (1.0 - 1e-9)) {
+                best = c;
+                best_lz = lz;
+            }
+        }
+        return best_lz;
+    }
+    // Other tiles, two regimes (measured with 32 x 8 tiles, ms per
     // step, 8 bubbles):
     //  * lattices too small to fill the GPU with 16-plane chunks are latency
     //    bound: one wave of two CTAs per SM with chunks of >= 8 planes

@@ -168,7 +168,7 @@ int arith_mode(const bubble_spec &spec);
 
 // Default z chunk of the fused kernel for a lattice.  FP32 16 x 16 tiles:
 // the chunk whose cheaper form is cheapest under column_stage_cost (params.h);
-// otherwise enough CTAs to fill the GPU while keeping each chunk's warm-up a
+// FP64: the cheapest under fp64_stage_cost; otherwise enough CTAs to fill the GPU while keeping each chunk's warm-up a
 // small fraction of its work.
 int default_chunk(const uint32_t grid[3], int ty, bool fp32);
 // z chunk of the pair form (stage_pair.cuh) where the caller set none: the
