@@ -188,14 +188,14 @@ __global__ void stage_ref_kernel(StageArgs<R> A, const V4<R> *__restrict__ prim,
         const V4<R> rp = sanitise(half_step(qp1, s_p1, R(-1)), P.p_floor, zmax2);
         V4<R> fm, fp;
         if (axis == 0) {
-            fm = hll_flux<0, R, false>(lm, rm, zmax2, P);
-            fp = hll_flux<0, R, false>(lp, rp, zmax2, P);
+            fm = hll_flux<0, R, false, kPlain, false>(lm, rm, zmax2, P);
+            fp = hll_flux<0, R, false, kPlain, false>(lp, rp, zmax2, P);
         } else if (axis == 1) {
-            fm = hll_flux<1, R, false>(lm, rm, zmax2, P);
-            fp = hll_flux<1, R, false>(lp, rp, zmax2, P);
+            fm = hll_flux<1, R, false, kPlain, false>(lm, rm, zmax2, P);
+            fp = hll_flux<1, R, false, kPlain, false>(lp, rp, zmax2, P);
         } else {
-            fm = hll_flux<2, R, false>(lm, rm, zmax2, P);
-            fp = hll_flux<2, R, false>(lp, rp, zmax2, P);
+            fm = hll_flux<2, R, false, kPlain, false>(lm, rm, zmax2, P);
+            fp = hll_flux<2, R, false, kPlain, false>(lp, rp, zmax2, P);
         }
         fd.x = fd.x + (fp.x - fm.x) * P.inv_dx;
         fd.y = fd.y + (fp.y - fm.y) * P.inv_dx;

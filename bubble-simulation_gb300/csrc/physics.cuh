@@ -84,6 +84,63 @@ BUBBLE_DEV float dot3_rn(float x, float y, float z) { return __fmaf_rn(z, z, __f
 BUBBLE_DEV double dot3_rn(double x, double y, double z) { return __fma_rn(z, z, __fma_rn(y, y, __dmul_rn(x, x))); }
 
 // ---------------------------------------------------------------------------
+//  FP64 comparisons on the integer pipe
+// ---------------------------------------------------------------------------
+// GB300 runs two FP64 operations per clock and SM, and a comparison, minimum
+// or maximum of doubles is one of them; on the bit patterns it is a few of the
+// integer pipe's 64 per clock.  Each returns what the FP64 operation does, a
+// NaN operand included.
+constexpr long long kInfBits = 0x7ff0000000000000ll;
+BUBBLE_DEV bool d_above(double a, double c) {  // a > c for c > 0
+    const long long x = __double_as_longlong(a);
+    return x > __double_as_longlong(c) && x <= kInfBits;
+}
+BUBBLE_DEV double d_max_pos(double a, double c) { return d_above(a, c) ? a : c; }  // fmax(a, c), c > 0
+BUBBLE_DEV double d_max_zero(double a) {                                            // fmax(a, 0)
+    const long long x = __double_as_longlong(a);
+    return x > 0 && x <= kInfBits ? a : 0.0;
+}
+BUBBLE_DEV double d_min_pos(double a, double c) {  // fmin(a, c) for a >= 0 (or NaN), c > 0
+    return __double_as_longlong(a) < __double_as_longlong(c) ? a : c;
+}
+template <typename R>
+BUBBLE_DEV R max_pos(R a, R c) {  // max(a, c) for c > 0
+    if constexpr (sizeof(R) == 8) return d_max_pos(a, c);
+    else return vmax(a, c);
+}
+template <typename R>
+BUBBLE_DEV R max_zero(R a) {  // max(a, 0)
+    if constexpr (sizeof(R) == 8) return d_max_zero(a);
+    else return vmax(a, R(0));
+}
+template <typename R>
+BUBBLE_DEV bool above(R a, R c) {  // a > c for c > 0
+    if constexpr (sizeof(R) == 8) return d_above(a, c);
+    else return a > c;
+}
+// order-preserving integer image of a double
+BUBBLE_DEV long long d_key(double a) {
+    const long long x = __double_as_longlong(a);
+    return x ^ ((x >> 63) & 0x7fffffffffffffffll);
+}
+BUBBLE_DEV bool d_nan(double a) { return (__double_as_longlong(a) & 0x7fffffffffffffffll) > kInfBits; }
+BUBBLE_DEV double d_min(double a, double b) { return d_nan(a) ? b : (d_nan(b) || d_key(a) <= d_key(b) ? a : b); }
+BUBBLE_DEV double d_max(double a, double b) { return d_nan(a) ? b : (d_nan(b) || d_key(a) >= d_key(b) ? a : b); }
+
+// Half of the MC-limited slope of limit_slope<double, false>: the minimum of
+// |dm + dp| / 4, |dm| and |dp| with their sign, 0 unless dm and dp have one.
+// Scaling by powers of two is exact, so q +- this is half_step's q +- s / 2.
+BUBBLE_DEV double d_half_slope(double dm, double dp) {
+    const unsigned long long sign = 0x8000000000000000ull;
+    const unsigned long long a = (unsigned long long)__double_as_longlong(dm), b = (unsigned long long)__double_as_longlong(dp);
+    const bool same = ((a ^ b) & sign) == 0 && (a & ~sign) != 0 && (b & ~sign) != 0 && !d_nan(dm) && !d_nan(dp);
+    const unsigned long long h = (unsigned long long)__double_as_longlong(0.25 * (dm + dp)) & ~sign;
+    const unsigned long long m0 = (a & ~sign) < (b & ~sign) ? (a & ~sign) : (b & ~sign);
+    const unsigned long long m = h < m0 ? h : m0;
+    return same ? __longlong_as_double((long long)(m | (a & sign))) : 0.0;
+}
+
+// ---------------------------------------------------------------------------
 //  Potential (shaders/potential.wgsl:38-47)
 // ---------------------------------------------------------------------------
 template <typename R>
@@ -126,7 +183,7 @@ BUBBLE_DEV R limit_slope(R dm, R dp) {
 // eos_prim_from_cons(eos_regularise(u)) -> (vx, vy, vz, p).
 template <typename R, bool FAST>
 BUBBLE_DEV V4<R> prim_from_cons(const V4<R> &u, const LatticeParams<R> &P) {
-    const R e_lab = vmax(u.x, P.e_floor);
+    const R e_lab = max_pos(u.x, P.e_floor);
     R zx = u.y, zy = u.z, zz = u.w;
     const R zcap = P.z_max * e_lab;
     if constexpr (FAST) {
@@ -148,17 +205,17 @@ BUBBLE_DEV V4<R> prim_from_cons(const V4<R> &u, const LatticeParams<R> &P) {
         return V4<R>{__fmul_rn(zx, inv), __fmul_rn(zy, inv), __fmul_rn(zz, inv), p};
     } else {
         const R zlen = sqrt(zx * zx + zy * zy + zz * zz);
-        if (zlen > zcap) {
+        if (above(zlen, zcap)) {
             const R s = zcap / vmax(zlen, R(1e-30));
             zx = zx * s;
             zy = zy * s;
             zz = zz * s;
         }
         const R z2 = zx * zx + zy * zy + zz * zz;
-        const R disc = vmax(R(4.0) * e_lab * e_lab - R(3.0) * z2, R(0.0));
+        const R disc = max_zero(R(4.0) * e_lab * e_lab - R(3.0) * z2);
         R p = (e_lab * e_lab - z2) / (e_lab + sqrt(disc));
-        p = vmax(p, P.p_floor);
-        const R s = vmax(e_lab + p, R(1e-30));
+        p = max_pos(p, P.p_floor);
+        const R s = max_pos(e_lab + p, R(1e-30));
         return V4<R>{zx / s, zy / s, zz / s, p};
     }
 }
@@ -532,10 +589,10 @@ BUBBLE_DEV V4<R> recover(const V4<R> &u, const LatticeParams<R> &P, R phi = R(0)
 // ---------------------------------------------------------------------------
 template <typename R>
 BUBBLE_DEV V4<R> sanitise(const V4<R> &q, R p_floor, R vmax2) {
-    const R p = vmax(q.w, p_floor);
+    const R p = max_pos(q.w, p_floor);
     R vx = q.x, vy = q.y, vz = q.z;
     const R v2 = vx * vx + vy * vy + vz * vz;
-    if (v2 > vmax2) {
+    if (above(v2, vmax2)) {
         const R s = sqrt(vmax2 / vmax(v2, R(1e-30)));
         vx = vx * s;
         vy = vy * s;
@@ -618,6 +675,13 @@ BUBBLE_DEV void face_states(const V4<R> &qm, const V4<R> &q, const V4<R> &qp, R 
         hi = v4of(p_fma(sa, bc2(0.5f), qa), p_fma(sb, bc2(0.5f), qb));
         lo.w = vmax(lo.w, p_floor);
         hi.w = vmax(hi.w, p_floor);
+    } else if constexpr (sizeof(R) == 8) {
+        // the velocity clamp is left to face_side, where |v|^2 is needed anyway
+        // (same values, one |v|^2 per face state instead of two)
+        const V4<R> s{d_half_slope(q.x - qm.x, qp.x - q.x), d_half_slope(q.y - qm.y, qp.y - q.y),
+                      d_half_slope(q.z - qm.z, qp.z - q.z), d_half_slope(q.w - qm.w, qp.w - q.w)};
+        lo = V4<R>{q.x - s.x, q.y - s.y, q.z - s.z, d_max_pos(q.w - s.w, p_floor)};
+        hi = V4<R>{q.x + s.x, q.y + s.y, q.z + s.z, d_max_pos(q.w + s.w, p_floor)};
     } else {
         const V4<R> s = limit_slope4<R, FAST>(v4_sub(q, qm), v4_sub(qp, q));
         lo = sanitise(half_step(q, s, R(-1)), p_floor, vmax2);
@@ -650,7 +714,9 @@ struct FaceSide {
 // with c_s^2 = c2; E = w W^2 - p and the fluxes as for the bag model.
 // THERMAL (FORM kThermal): w = e(T, phi) + p with T = eos_temperature(p, phi)
 // and c_s^2(T, phi), phi the field value of the state's own cell.
-template <int AXIS, typename R, bool FAST, int FORM = kPlain>
+// RAW: the states' velocities are not clamped yet (face_states leaves that to
+// this point in the fast arithmetic and in FP64).
+template <int AXIS, typename R, bool FAST, int FORM = kPlain, bool RAW = FAST || sizeof(R) == 8>
 BUBBLE_DEV FaceSide<R> face_side(const V4<R> &q, R zmax2, const LatticeParams<R> &P, R phi = R(0)) {
     constexpr bool PERT = FORM == kPert;
     static_assert(!FAST || FORM == kPlain || FORM == kMixed, "the other fast forms run in the pair form");
@@ -675,7 +741,19 @@ BUBBLE_DEV FaceSide<R> face_side(const V4<R> &q, R zmax2, const LatticeParams<R>
             v2raw = dot3_rn(vx, vy, vz);
         }
     }
-    const R v2 = vmin(v2raw, zmax2);
+    R v2;
+    if constexpr (sizeof(R) == 8) {
+        if (RAW && d_above(v2raw, zmax2)) {  // the velocity half of sanitise
+            const R sc = sqrt(zmax2 / vmax(v2raw, R(1e-30)));
+            vx = vx * sc;
+            vy = vy * sc;
+            vz = vz * sc;
+            v2raw = vx * vx + vy * vy + vz * vz;
+        }
+        v2 = d_min_pos(v2raw, zmax2);
+    } else {
+        v2 = vmin(v2raw, zmax2);
+    }
     const R vd = AXIS == 0 ? vx : (AXIS == 1 ? vy : vz);
     if constexpr (FORM == kGamma || FORM == kThermal) {
         R cs2, enth;
@@ -731,7 +809,9 @@ BUBBLE_DEV FaceSide<R> face_side(const V4<R> &q, R zmax2, const LatticeParams<R>
         s.u = V4<R>{PERT ? w * v2 + R(3.0) * p : w - p, w * vx, w * vy, w * vz};
         const R cs = sqrt(cs2);
         const R denom = R(1.0) - v2 * cs2;
-        const R rad = vmax((R(1.0) - v2) * (R(1.0) - vd * vd - cs2 * (v2 - vd * vd)), R(0.0));
+        R rad = (R(1.0) - v2) * (R(1.0) - vd * vd - cs2 * (v2 - vd * vd));
+        if constexpr (sizeof(R) == 8) rad = d_max_zero(rad);
+        else rad = vmax(rad, R(0.0));
         const R a = vd * (R(1.0) - cs2) / denom;
         const R b = cs * sqrt(rad) / denom;
         s.lm = a - b;
@@ -747,14 +827,21 @@ BUBBLE_DEV FaceSide<R> face_side(const V4<R> &q, R zmax2, const LatticeParams<R>
 
 // hll_flux(q_l, phi_l, q_r, phi_r, axis).  The phi arguments reach only the
 // EOS functions; the forms whose EOS ignores phi pass 0.
-template <int AXIS, typename R, bool FAST, int FORM = kPlain>
+template <int AXIS, typename R, bool FAST, int FORM = kPlain, bool RAW = FAST || sizeof(R) == 8>
 BUBBLE_DEV V4<R> hll_flux(const V4<R> &ql, const V4<R> &qr, R zmax2, const LatticeParams<R> &P, R phi_l = R(0),
                           R phi_r = R(0)) {
-    const FaceSide<R> L = face_side<AXIS, R, FAST, FORM>(ql, zmax2, P, phi_l);
-    const FaceSide<R> Rt = face_side<AXIS, R, FAST, FORM>(qr, zmax2, P, phi_r);
-    const R s_min = vmin(vmin(L.lm, Rt.lm), R(0.0));
-    const R s_max = vmax(vmax(L.lp, Rt.lp), R(0.0));
-    const R den = vmax(s_max - s_min, R(1e-12));
+    const FaceSide<R> L = face_side<AXIS, R, FAST, FORM, RAW>(ql, zmax2, P, phi_l);
+    const FaceSide<R> Rt = face_side<AXIS, R, FAST, FORM, RAW>(qr, zmax2, P, phi_r);
+    R s_min, s_max, den;
+    if constexpr (sizeof(R) == 8) {
+        s_min = d_min(d_min(L.lm, Rt.lm), R(0.0));
+        s_max = d_max(d_max(L.lp, Rt.lp), R(0.0));
+        den = d_max_pos(s_max - s_min, R(1e-12));
+    } else {
+        s_min = vmin(vmin(L.lm, Rt.lm), R(0.0));
+        s_max = vmax(vmax(L.lp, Rt.lp), R(0.0));
+        den = vmax(s_max - s_min, R(1e-12));
+    }
     const R smm = s_min * s_max;
     if constexpr (FAST) {
         const R inv = rcp_approx(den);

@@ -99,13 +99,16 @@ BUBBLE_DEV void combine_cell(const StageArgs<R> &A, const LatticeParams<R> &P, u
                              const V4<R> &fym, const V4<R> &fyp, const V4<R> &fzm, const V4<R> &fzp,
                              const V2<R> &pf, const V4<R> &pu, const V2<R> &pfn, const V4<R> &pun) {
     const R pi0 = pf.y;
-    R lap_sum = R(0), gx, gy, gz;
-    lap_sum = lap_sum + (phxm + phxp - R(2.0) * phi0);
-    gx = R(0.5) * (phxp - phxm) * P.inv_dx;
-    lap_sum = lap_sum + (phym + phyp - R(2.0) * phi0);
-    gy = R(0.5) * (phyp - phym) * P.inv_dx;
-    lap_sum = lap_sum + (phzm + phzp - R(2.0) * phi0);
-    gz = R(0.5) * (phzp - phzm) * P.inv_dx;
+    // x * inv_dx; in FP64 not multiplied where that is 1 (the default spacing)
+    const bool unit = sizeof(R) == 8 && P.inv_dx == R(1.0);
+    auto over_dx = [&](R x) { return unit ? x : x * P.inv_dx; };
+    const R two_phi = R(2.0) * phi0;
+    R lap_sum = phxm + phxp - two_phi;
+    const R gx = over_dx(R(0.5) * (phxp - phxm));
+    lap_sum = lap_sum + (phym + phyp - two_phi);
+    const R gy = over_dx(R(0.5) * (phyp - phym));
+    lap_sum = lap_sum + (phzm + phzp - two_phi);
+    const R gz = over_dx(R(0.5) * (phzp - phzm));
     V4<R> fd;
     if constexpr (FAST && sizeof(R) == 4) {
         // ((dx + dy) + dz) / dx on the (x, y) and (z, w) halves
@@ -117,21 +120,12 @@ BUBBLE_DEV void combine_cell(const StageArgs<R> &A, const LatticeParams<R> &P, u
                                 bc2(P.inv_dx));
         fd = v4of(fa, fb);
     } else {
-        fd = V4<R>{R(0), R(0), R(0), R(0)};
-        fd.x = fd.x + (fxp.x - fxm.x) * P.inv_dx;
-        fd.y = fd.y + (fxp.y - fxm.y) * P.inv_dx;
-        fd.z = fd.z + (fxp.z - fxm.z) * P.inv_dx;
-        fd.w = fd.w + (fxp.w - fxm.w) * P.inv_dx;
-        fd.x = fd.x + (fyp.x - fym.x) * P.inv_dx;
-        fd.y = fd.y + (fyp.y - fym.y) * P.inv_dx;
-        fd.z = fd.z + (fyp.z - fym.z) * P.inv_dx;
-        fd.w = fd.w + (fyp.w - fym.w) * P.inv_dx;
-        fd.x = fd.x + (fzp.x - fzm.x) * P.inv_dx;
-        fd.y = fd.y + (fzp.y - fzm.y) * P.inv_dx;
-        fd.z = fd.z + (fzp.z - fzm.z) * P.inv_dx;
-        fd.w = fd.w + (fzp.w - fzm.w) * P.inv_dx;
+        fd.x = over_dx(fxp.x - fxm.x) + over_dx(fyp.x - fym.x) + over_dx(fzp.x - fzm.x);
+        fd.y = over_dx(fxp.y - fxm.y) + over_dx(fyp.y - fym.y) + over_dx(fzp.y - fzm.y);
+        fd.z = over_dx(fxp.z - fxm.z) + over_dx(fyp.z - fym.z) + over_dx(fzp.z - fzm.z);
+        fd.w = over_dx(fxp.w - fxm.w) + over_dx(fyp.w - fym.w) + over_dx(fzp.w - fzm.w);
     }
-    const R laplacian = lap_sum * P.inv_dx * P.inv_dx;
+    const R laplacian = over_dx(over_dx(lap_sum));
     const R vv = q0.x * q0.x + q0.y * q0.y + q0.z * q0.z;
     R gam;
     if constexpr (FAST) gam = rsqrt_approx(vmax(R(1.0) - vv, R(1e-12)));
