@@ -20,6 +20,11 @@
 namespace bubble {
 namespace dev {
 
+// Start of a kernel launched as a programmatic dependent: waits until the
+// launches before it have completed and their stores are visible.  Does
+// nothing in a plain launch.
+BUBBLE_DEV void await_previous_launch() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 // wrap1 (shaders/common.wgsl:80-89): reach <= 2 with n >= 8, one add suffices.
 BUBBLE_DEV int wrap1(int i, int n) {
     int r = i;
@@ -86,6 +91,7 @@ template <typename R>
 __global__ void __launch_bounds__(256) nucleate_kernel(V2<R> *__restrict__ field,
                                                         const __grid_constant__ BubbleBatch batch,
                                                         LatticeParams<R> P) {
+    await_previous_launch();
     __shared__ int kept[kNucleateBatch];
     __shared__ int n_kept;
     const int bx = blockIdx.x * kNucBx, by = blockIdx.y * kNucBy, bz = blockIdx.z * kNucBz;
@@ -245,6 +251,24 @@ __global__ void stage_ref_kernel(StageArgs<R> A, const V4<R> *__restrict__ prim,
 // FP64.  Every block writes its partial to `partials`; the last block to
 // finish (ticket counter) folds them in a fixed order, writes `out` and
 // re-arms the counter, so the result does not depend on block timing.
+//
+// Work item: 256 cells of a plane, one per thread, marched through a chunk of
+// z planes with phi of the planes around z carried in registers, so a cell's
+// position is decoded once per item and the field and fluid are read once.
+//
+// What bounded it (3.24 ms a report at 512^3, 0.47 ms of traffic): IEEE
+// divisions with zero or tiny numerators, which leave the fast path
+// (div_scaled: 2.27 -> 1.29 ms at four blocks per SM), residency (2.07 -> 1.29
+// ms) and the FP64 pipe, which adds two doubles per clock and SM (0.4 ms).  An
+// FP32 state's terms are summed over a chunk as unevaluated pairs hi + lo
+// (Knuth's TwoSum; lo collects the exact rounding errors of hi) and the pair
+// is added in FP64 once per chunk; cells of the broken phase are counted.  lo
+// is a sum of at most 32 terms below 2^-24 hi, so a chunk's pair is within
+// 2^-44 of exact, unbiased, and the total over many chunks well below that
+// (the fluid energies of 64^3 to 256^3 states sum to the correctly rounded
+// double).  The largest speed is taken from the largest |v|^2 (sqrt is
+// monotone).  Now 1.27 ms at 512^3, bound by instruction issue; 256^3 0.59 ->
+// 0.21 ms, 128^3 96 -> 60 us.
 constexpr int kDiagThreads = 256;
 constexpr int kDiagMaxBlocks = 1024;
 
@@ -262,70 +286,164 @@ BUBBLE_DEV double warp_sum(double v) {
     return v;
 }
 
+constexpr int kDiagBlocksPerSm = 4;  // at 512^3: 2.07 ms with 3, 1.29 with 4, 1.40 with 5, 1.66 with 8
+
+// Planes of a chunk: about two items per SM on small lattices (one round of
+// blocks: 64^3 58 us a report at one plane, 39 at four), at most 32 planes.
+BUBBLE_HD int diag_planes(uint64_t nx, uint64_t ny, uint64_t nz) {
+    const uint64_t groups = (nx * ny + kDiagThreads - 1) / kDiagThreads;
+    const uint64_t lz = (groups * nz + 299) / 300;
+    return lz > 32 ? 32 : (int)lz;
+}
+
+// A sum of FP32 terms as hi + lo, or of doubles.
+template <typename R>
+struct TermSum {
+    R hi = R(0), lo = R(0);
+    BUBBLE_DEV void add(R x) {
+        if constexpr (sizeof(R) == 4) {
+            const R s = hi + x;
+            const R b = s - hi;
+            lo = lo + ((hi - (s - b)) + (x - b));
+            hi = s;
+        } else {
+            hi += x;
+        }
+    }
+    BUBBLE_DEV double take() {
+        const double v = (double)hi + (double)lo;
+        hi = lo = R(0);
+        return v;
+    }
+};
+
+// a / b for a normal b > 0, kept on IEEE division's fast path: a zero or tiny a,
+// common in the fluid at rest ahead of the walls, goes to a subroutine there and
+// splits its warp.  The scaling is exact; a quotient below 2^-126 is rounded
+// twice, and every such quotient is squared or added to the energy density,
+// where it is far below rounding.
+BUBBLE_DEV float div_scaled(float a, float b) {
+    const bool small = fabsf(a) < 1.0f;
+    const float n = a == 0.0f ? 1.0f : a * (small ? 0x1p48f : 1.0f);
+    const float q = n / b * (small ? 0x1p-48f : 1.0f);
+    return a == 0.0f ? a : q;
+}
+
+// recover<R, false, MIXED>(u, P, phi) with those divisions.
 template <typename R, int MIXED>
-__global__ void __launch_bounds__(kDiagThreads)
+BUBBLE_DEV V4<R> diag_recover(const V4<R> &u, const LatticeParams<R> &P, R phi) {
+    if constexpr (sizeof(R) == 4 && (MIXED == kPlain || MIXED == kMixed || MIXED == kPert)) {
+        const float de = vmax(u.x, P.e_floor);
+        const float e_lab = MIXED == kPert ? P.e_bg + de : de;
+        float zx = u.y, zy = u.z, zz = u.w;
+        const float zcap = P.z_max * e_lab;
+        V4<float> q;
+        if constexpr (MIXED == kPert) {
+            const float z2 = capped_z2(zx, zy, zz, zcap);
+            const float sq = sqrt(vmax(4.0f * e_lab * e_lab - 3.0f * z2, 0.0f));
+            const float dp = vmax(div_scaled(de, 3.0f) - div_scaled(z2, sq + 2.0f * e_lab), P.p_floor);
+            const float d = vmax(e_lab + P.p_bg + dp, 1e-30f);
+            q = V4<float>{div_scaled(zx, d), div_scaled(zy, d), div_scaled(zz, d), dp};
+        } else {
+            const PrimParts<float> r = prim_parts(e_lab, zx, zy, zz, zcap, P);
+            q = V4<float>{div_scaled(r.zx, r.s), div_scaled(r.zy, r.s), div_scaled(r.zz, r.s), r.p};
+        }
+        if constexpr (MIXED != kPlain) {
+            if (q.x * q.x + q.y * q.y + q.z * q.z > 8.0f / 9.0f) return recover<R, false, MIXED>(u, P, phi);
+        }
+        return q;
+    } else {
+        return recover<R, false, MIXED>(u, P, phi);
+    }
+}
+// potential(phi, P) likewise
+template <typename R>
+BUBBLE_DEV R diag_potential(R phi, const LatticeParams<R> &P) {
+    if constexpr (sizeof(R) == 4) {
+        const R p2 = phi * phi;
+        return 0.5f * P.m2 * p2 - div_scaled(P.delta * p2 * phi, 3.0f) + 0.25f * P.lambda * p2 * p2;
+    } else {
+        return potential(phi, P);
+    }
+}
+
+template <typename R, int MIXED>
+__global__ void __launch_bounds__(kDiagThreads, kDiagBlocksPerSm)
     diag_kernel(const V2<R> *__restrict__ field, const V4<R> *__restrict__ fluid,
                 LatticeParams<R> P, DiagPartial *__restrict__ partials,
                 unsigned int *__restrict__ ticket, DiagResult *__restrict__ out) {
+    await_previous_launch();
     const uint64_t n = (uint64_t)P.nx * P.ny * P.nz;
-    const uint64_t xy = (uint64_t)P.nx * P.ny;
+    const uint32_t plane = (uint32_t)P.nx * (uint32_t)P.ny;
+    const uint32_t groups = (plane + kDiagThreads - 1) / kDiagThreads;
+    const int lz = diag_planes(P.nx, P.ny, P.nz);
+    const uint32_t items = groups * (uint32_t)((P.nz + lz - 1) / lz);
     double acc[4] = {0.0, 0.0, 0.0, 0.0};
-    float vmaxv = 0.0f;
+    R v2max = R(0);
     uint32_t bad = 0;
-    const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
-    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
-        const int z = (int)(i / xy);
-        const int rem = (int)(i - (uint64_t)z * xy);
-        const int y = rem / P.nx;
-        const int x = rem - y * P.nx;
-        const V2<R> f = field[i];
-        const R phi = f.x, pi = f.y;
-        R grad2 = R(0);
-        {
-            const R d = R(0.5) *
-                        (field[cell_index(wrap1(x + 1, P.nx), y, z, P)].x -
-                         field[cell_index(wrap1(x - 1, P.nx), y, z, P)].x) *
-                        P.inv_dx;
-            grad2 = grad2 + d * d;
+    for (uint32_t it = blockIdx.x; it < items; it += gridDim.x) {
+        const uint32_t chunk = it / groups;
+        const uint32_t c = (it - chunk * groups) * kDiagThreads + threadIdx.x;
+        if (c >= plane) continue;
+        const int y = (int)(c / (uint32_t)P.nx), x = (int)(c - (uint32_t)y * (uint32_t)P.nx);
+        // in-plane neighbours, periodic
+        const uint32_t cxp = x + 1 < P.nx ? c + 1 : c + 1 - P.nx, cxm = x > 0 ? c - 1 : c - 1 + P.nx;
+        const uint32_t cyp = y + 1 < P.ny ? c + P.nx : c + P.nx - plane, cym = y > 0 ? c - P.nx : c - P.nx + plane;
+        const int z0 = (int)chunk * lz, z1 = min(z0 + lz, P.nz);
+        // cell indices fit 32 bits
+        R phi_m = field[(uint32_t)wrap1(z0 - 1, P.nz) * plane + c].x;
+        V2<R> f = field[(uint32_t)z0 * plane + c];
+        TermSum<R> s_total, s_kinetic, s_e;
+        uint32_t broken = 0;
+#pragma unroll 1
+        for (int z = z0; z < z1; ++z) {
+            const uint32_t pl = (uint32_t)z * plane;
+            const V2<R> f_p = field[(uint32_t)wrap1(z + 1, P.nz) * plane + c];
+            const V4<R> u = fluid[pl + c];
+            const R phi = f.x, pi = f.y;
+            R grad2 = R(0);
+            {
+                const R d = R(0.5) * (field[pl + cxp].x - field[pl + cxm].x) * P.inv_dx;
+                grad2 = grad2 + d * d;
+            }
+            {
+                const R d = R(0.5) * (field[pl + cyp].x - field[pl + cym].x) * P.inv_dx;
+                grad2 = grad2 + d * d;
+            }
+            {
+                const R d = R(0.5) * (f_p.x - phi_m) * P.inv_dx;
+                grad2 = grad2 + d * d;
+            }
+            // In the perturbation form e_lab is max(E, e_floor) - e_bg: the sums of
+            // e_total and e_lab then miss N e_bg, which the host adds in FP64.
+            const R e_lab = vmax(u.x, P.e_floor);
+            const V4<R> q = diag_recover<R, MIXED>(u, P, phi);
+            const R v2 = q.x * q.x + q.y * q.y + q.z * q.z;
+            // the thermal form's field holds V(phi, 0); the rest of V(phi, T) is in E
+            R pot;
+            if constexpr (MIXED == kThermal) pot = thermal_potential0(phi, P);
+            else pot = diag_potential(phi, P);
+            const R e_total = R(0.5) * pi * pi + R(0.5) * grad2 + pot + e_lab;
+            R kinetic;
+            if constexpr (MIXED == kPert) kinetic = ((e_lab + q.w) + (P.e_bg + P.p_bg)) * v2;
+            else kinetic = (e_lab + q.w) * v2;
+            s_total.add(e_total);
+            s_kinetic.add(kinetic);
+            s_e.add(e_lab);
+            broken += phi > R(0.5) * P.phi_b ? 1u : 0u;
+            v2max = vmax(v2max, v2);
+            // max(E, e_floor) hides a NaN in E, so the raw state is checked too.
+            if (!isfinite(e_total) || !isfinite(v2) || !isfinite(f.x + f.y + u.x + u.y + u.z + u.w)) bad = 1;
+            phi_m = phi;
+            f = f_p;
         }
-        {
-            const R d = R(0.5) *
-                        (field[cell_index(x, wrap1(y + 1, P.ny), z, P)].x -
-                         field[cell_index(x, wrap1(y - 1, P.ny), z, P)].x) *
-                        P.inv_dx;
-            grad2 = grad2 + d * d;
-        }
-        {
-            const R d = R(0.5) *
-                        (field[cell_index(x, y, wrap1(z + 1, P.nz), P)].x -
-                         field[cell_index(x, y, wrap1(z - 1, P.nz), P)].x) *
-                        P.inv_dx;
-            grad2 = grad2 + d * d;
-        }
-        const V4<R> u = fluid[i];
-        // In the perturbation form e_lab is max(E, e_floor) - e_bg: the sums of
-        // e_total and e_lab then miss N e_bg, which the host adds in FP64.
-        const R e_lab = vmax(u.x, P.e_floor);
-        const V4<R> q = recover<R, false, MIXED>(u, P, phi);
-        const R v2 = q.x * q.x + q.y * q.y + q.z * q.z;
-        // the thermal form's field holds V(phi, 0); the rest of V(phi, T) is in E
-        R pot;
-        if constexpr (MIXED == kThermal) pot = thermal_potential0(phi, P);
-        else pot = potential(phi, P);
-        const R e_total = R(0.5) * pi * pi + R(0.5) * grad2 + pot + e_lab;
-        const R broken = phi > R(0.5) * P.phi_b ? R(1.0) : R(0.0);
-        R kinetic;
-        if constexpr (MIXED == kPert) kinetic = ((e_lab + q.w) + (P.e_bg + P.p_bg)) * v2;
-        else kinetic = (e_lab + q.w) * v2;
-        acc[0] += (double)e_total;
+        acc[0] += s_total.take();
         acc[1] += (double)broken;
-        acc[2] += (double)kinetic;
-        acc[3] += (double)e_lab;
-        const float vl = (float)sqrt(v2);
-        // max(E, e_floor) hides a NaN in E, so the raw state is checked too.
-        if (!isfinite(e_total) || !isfinite(vl) || !isfinite(f.x + f.y + u.x + u.y + u.z + u.w)) bad = 1;
-        vmaxv = fmaxf(vmaxv, vl);
+        acc[2] += s_kinetic.take();
+        acc[3] += s_e.take();
     }
+    float vmaxv = (float)sqrt(v2max);
+    if (!isfinite(vmaxv)) bad = 1;
     __shared__ double sh[kDiagThreads / 32][4];
     __shared__ float shm[kDiagThreads / 32];
     __shared__ uint32_t shb[kDiagThreads / 32];
@@ -403,11 +521,13 @@ __global__ void __launch_bounds__(kDiagThreads)
     }
 }
 
-inline int diag_blocks(uint64_t n) {
-    uint64_t b = (n + kDiagThreads - 1) / kDiagThreads;
-    if (b > (uint64_t)kDiagMaxBlocks) b = kDiagMaxBlocks;
-    if (b < 1) b = 1;
-    return (int)b;
+// One block per item, at most the blocks that `sms` SMs hold.
+inline int diag_blocks(uint64_t nx, uint64_t ny, uint64_t nz, int sms) {
+    const uint64_t lz = (uint64_t)diag_planes(nx, ny, nz);
+    const uint64_t items = (nx * ny + kDiagThreads - 1) / kDiagThreads * ((nz + lz - 1) / lz);
+    uint64_t most = (uint64_t)kDiagBlocksPerSm * (uint64_t)(sms > 0 ? sms : 1);
+    if (most > (uint64_t)kDiagMaxBlocks) most = kDiagMaxBlocks;
+    return (int)(items < most ? items : most);
 }
 
 }  // namespace dev

@@ -37,7 +37,6 @@ cudaError_t diag_f32(const V2<float> *field, const V4<float> *fluid,
 }
 
 size_t diag_partials_bytes() { return sizeof(dev::DiagPartial) * dev::kDiagMaxBlocks; }
-int diag_blocks_for(uint64_t cells) { return dev::diag_blocks(cells); }
 
 }  // namespace launch
 }  // namespace bubble

@@ -48,7 +48,6 @@ cudaError_t diag_f64(const V2<double> *field, const V4<double> *fluid,
 
 // Scratch of the diagnostics reduction: partials + ticket.
 size_t diag_partials_bytes();
-int diag_blocks_for(uint64_t cells);
 
 // ---- fused stage kernel, column form (stage_column.cuh) -----------------------
 // `maps` are the tensor maps of the stage input slot (tma.h); `tma_ok` says

@@ -48,6 +48,32 @@ inline cudaError_t ensure_smem(Kernel k, size_t bytes) {
     return ensure_smem_ptr(reinterpret_cast<const void *>(k), bytes);
 }
 
+// Stage, nucleation and diagnostics launches are programmatic dependents: the next launch
+// is set up while the one before still runs and its CTAs wait for that one's
+// end in the kernel (await_previous_launch), so the gap between two launches
+// shrinks by about 2 us (per step of three stages: 32^3 24.7 -> 17.4 us, 64^3
+// 43.1 -> 37.3, 128^3 170 -> 161).  No kernel releases its dependents early:
+// CTAs placed beside a running grid land unevenly on the SMs (96^3 92 -> 107
+// us).  A capturing stream gets plain launches.
+template <typename Kernel, typename... Args>
+cudaError_t launch_dependent(Kernel k, dim3 grid, int threads, size_t smem, cudaStream_t s, Args... args) {
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    cudaError_t e = cudaStreamIsCapturing(s, &cap);
+    if (e != cudaSuccess) return e;
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3((unsigned)threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cfg.attrs = &attr;
+    cfg.numAttrs = cap == cudaStreamCaptureStatusNone ? 1 : 0;
+    e = cudaLaunchKernelEx(&cfg, k, args...);
+    return e != cudaSuccess ? e : cudaGetLastError();
+}
+
 template <typename R>
 cudaError_t init(V2<R> *field, V4<R> *fluid, uint64_t n, R e_ref, cudaStream_t s) {
     dev::init_kernel<R><<<grid_for(n, 256), 256, 0, s>>>(field, fluid, n, e_ref);
@@ -64,8 +90,8 @@ cudaError_t nucleate(V2<R> *field, const V4<float> *bubbles, int count, const La
         batch.count = count - first < dev::kNucleateBatch ? count - first : dev::kNucleateBatch;
         batch._pad[0] = batch._pad[1] = batch._pad[2] = 0;
         for (int k = 0; k < batch.count; ++k) batch.b[k] = bubbles[first + k];
-        dev::nucleate_kernel<R><<<grid, dev::kNucBx * dev::kNucBy, 0, s>>>(field, batch, P);
-        cudaError_t e = cudaGetLastError();
+        const cudaError_t e =
+            launch_dependent(dev::nucleate_kernel<R>, grid, dev::kNucBx * dev::kNucBy, 0, s, field, batch, P);
         if (e != cudaSuccess) return e;
     }
     return cudaSuccess;
@@ -86,32 +112,6 @@ cudaError_t stage_ref(const StageArgs<R> &A, const V4<R> *prim, const LatticePar
     return cudaGetLastError();
 }
 
-// Stage launches are programmatic dependents of one another: the next launch
-// is set up while the one before still runs and its CTAs wait for that one's
-// end in the kernel (await_previous_launch), so the gap between two launches
-// shrinks by about 2 us (per step of three stages: 32^3 24.7 -> 17.4 us, 64^3
-// 43.1 -> 37.3, 128^3 170 -> 161).  No kernel releases its dependents early:
-// CTAs placed beside a running grid land unevenly on the SMs (96^3 92 -> 107
-// us).  A capturing stream gets plain launches.
-template <typename Kernel, typename... Args>
-cudaError_t launch_stage(Kernel k, dim3 grid, int threads, size_t smem, cudaStream_t s, Args... args) {
-    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-    cudaError_t e = cudaStreamIsCapturing(s, &cap);
-    if (e != cudaSuccess) return e;
-    cudaLaunchAttribute attr;
-    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr.val.programmaticStreamSerializationAllowed = 1;
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = grid;
-    cfg.blockDim = dim3((unsigned)threads);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = s;
-    cfg.attrs = &attr;
-    cfg.numAttrs = cap == cudaStreamCaptureStatusNone ? 1 : 0;
-    e = cudaLaunchKernelEx(&cfg, k, args...);
-    return e != cudaSuccess ? e : cudaGetLastError();
-}
-
 template <typename R, bool FAST, int FORM, int TY, bool LEAN = false>
 cudaError_t stage_column(const StageArgs<R> &A, const LatticeParams<R> &P, int lz, const StageMaps &maps, int tma_ok,
                      int *status, cudaStream_t s) {
@@ -123,7 +123,7 @@ cudaError_t stage_column(const StageArgs<R> &A, const LatticeParams<R> &P, int l
     const int ntx = (P.nx + L::TX - 1) / L::TX, nty = (P.ny + TY - 1) / TY;
     const int nzc = (P.nz + lz - 1) / lz;
     dim3 grid(ntx * nty, nzc);
-    return launch_stage(k, grid, L::NT, L::bytes, s, A, P, lz, maps, tma_ok, status);
+    return launch_dependent(k, grid, L::NT, L::bytes, s, A, P, lz, maps, tma_ok, status);
 }
 
 // A stage launch in the pair form (stage_pair.cuh).
@@ -136,7 +136,7 @@ cudaError_t stage_pair(const StageArgs<float> &A, const LatticeParams<float> &P,
     if (e != cudaSuccess) return e;
     if (lz < 1) lz = 1;
     const dim3 grid(((P.nx + 15) / 16) * ((P.ny + 15) / 16), (P.nz + lz - 1) / lz);
-    return launch_stage(k, grid, L::NT, L::bytes, s, A, P, lz, maps, tma_ok, status);
+    return launch_dependent(k, grid, L::NT, L::bytes, s, A, P, lz, maps, tma_ok, status);
 }
 
 // Whether a 16 x 16 FP32 launch of the column kernel takes the shared form: on request, or
@@ -172,11 +172,12 @@ cudaError_t stage_column16(const StageArgs<float> &A, const LatticeParams<float>
 template <typename R, int MIXED>
 cudaError_t diag(const V2<R> *field, const V4<R> *fluid, const LatticeParams<R> &P,
                  void *partials, unsigned int *ticket, DiagResult *out, cudaStream_t s) {
-    const uint64_t n = (uint64_t)P.nx * P.ny * P.nz;
-    const int blocks = dev::diag_blocks(n);
-    dev::diag_kernel<R, MIXED><<<blocks, dev::kDiagThreads, 0, s>>>(
-        field, fluid, P, reinterpret_cast<dev::DiagPartial *>(partials), ticket, out);
-    return cudaGetLastError();
+    int device = 0, sms = 0;
+    cudaGetDevice(&device);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
+    const int blocks = dev::diag_blocks(P.nx, P.ny, P.nz, sms);
+    return launch_dependent(dev::diag_kernel<R, MIXED>, dim3((unsigned)blocks), dev::kDiagThreads, 0, s, field, fluid, P,
+                            reinterpret_cast<dev::DiagPartial *>(partials), ticket, out);
 }
 
 }  // namespace launch_detail

@@ -180,6 +180,38 @@ BUBBLE_DEV R limit_slope(R dm, R dp) {
 // ---------------------------------------------------------------------------
 //  Bag EOS (shaders/eos.wgsl:94-123): conserved -> primitive
 // ---------------------------------------------------------------------------
+// Strict recovery up to its last divisions: the regularised Z, p and s = E +
+// p; v = Z / s.
+template <typename R>
+struct PrimParts {
+    R zx, zy, zz, p, s;
+};
+// |Z|^2 capped at zcap^2, Z scaled with it.  A |Z|^2 a hundredth below the cap's
+// square decides the comparison without the root.
+template <typename R>
+BUBBLE_DEV R capped_z2(R &zx, R &zy, R &zz, R zcap) {
+    R z2 = zx * zx + zy * zy + zz * zz;
+    if (above(z2, R(0.99) * (zcap * zcap))) {
+        const R zlen = sqrt(z2);
+        if (above(zlen, zcap)) {
+            const R s = zcap / vmax(zlen, R(1e-30));
+            zx = zx * s;
+            zy = zy * s;
+            zz = zz * s;
+            z2 = zx * zx + zy * zy + zz * zz;
+        }
+    }
+    return z2;
+}
+template <typename R>
+BUBBLE_DEV PrimParts<R> prim_parts(R e_lab, R zx, R zy, R zz, R zcap, const LatticeParams<R> &P) {
+    const R z2 = capped_z2(zx, zy, zz, zcap);
+    const R disc = max_zero(R(4.0) * e_lab * e_lab - R(3.0) * z2);
+    R p = (e_lab * e_lab - z2) / (e_lab + sqrt(disc));
+    p = max_pos(p, P.p_floor);
+    return PrimParts<R>{zx, zy, zz, p, max_pos(e_lab + p, R(1e-30))};
+}
+
 // eos_prim_from_cons(eos_regularise(u)) -> (vx, vy, vz, p).
 template <typename R, bool FAST>
 BUBBLE_DEV V4<R> prim_from_cons(const V4<R> &u, const LatticeParams<R> &P) {
@@ -204,19 +236,8 @@ BUBBLE_DEV V4<R> prim_from_cons(const V4<R> &u, const LatticeParams<R> &P) {
         const R inv = rcp_approx(vmax(__fadd_rn(e_lab, p), R(1e-30)));
         return V4<R>{__fmul_rn(zx, inv), __fmul_rn(zy, inv), __fmul_rn(zz, inv), p};
     } else {
-        const R zlen = sqrt(zx * zx + zy * zy + zz * zz);
-        if (above(zlen, zcap)) {
-            const R s = zcap / vmax(zlen, R(1e-30));
-            zx = zx * s;
-            zy = zy * s;
-            zz = zz * s;
-        }
-        const R z2 = zx * zx + zy * zy + zz * zz;
-        const R disc = max_zero(R(4.0) * e_lab * e_lab - R(3.0) * z2);
-        R p = (e_lab * e_lab - z2) / (e_lab + sqrt(disc));
-        p = max_pos(p, P.p_floor);
-        const R s = max_pos(e_lab + p, R(1e-30));
-        return V4<R>{zx / s, zy / s, zz / s, p};
+        const PrimParts<R> r = prim_parts(e_lab, zx, zy, zz, zcap, P);
+        return V4<R>{r.zx / r.s, r.zy / r.s, r.zz / r.s, r.p};
     }
 }
 
@@ -309,14 +330,7 @@ BUBBLE_DEV V4<R> prim_from_cons_pert(const V4<R> &u, const LatticeParams<R> &P) 
         const R inv = rcp_approx(vmax(__fadd_rn(__fadd_rn(e_lab, P.p_bg), dp), R(1e-30)));
         return V4<R>{__fmul_rn(zx, inv), __fmul_rn(zy, inv), __fmul_rn(zz, inv), dp};
     } else {
-        const R zlen = sqrt(zx * zx + zy * zy + zz * zz);
-        if (zlen > zcap) {
-            const R sc = zcap / vmax(zlen, R(1e-30));
-            zx = zx * sc;
-            zy = zy * sc;
-            zz = zz * sc;
-        }
-        const R z2 = zx * zx + zy * zy + zz * zz;
+        const R z2 = capped_z2(zx, zy, zz, zcap);
         const R sq = sqrt(vmax(R(4.0) * e_lab * e_lab - R(3.0) * z2, R(0.0)));
         R dp = de / R(3.0) - z2 / (sq + R(2.0) * e_lab);
         dp = vmax(dp, P.p_floor);

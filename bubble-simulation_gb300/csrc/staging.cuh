@@ -99,11 +99,6 @@ BUBBLE_DEV void cp_async_v2(V2<R> *dst, const V2<R> *src) {
     else cp_async_16(dst, src);
 }
 
-// Start of a kernel launched as a programmatic dependent: waits until the
-// launches before it have completed and their stores are visible.  Does
-// nothing in a plain launch.
-BUBBLE_DEV void await_previous_launch() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-
 constexpr int pad32(int n) { return (n + 31) / 32 * 32; }
 constexpr int round_up(int n, int m) { return (n + m - 1) / m * m; }
 constexpr size_t align128(size_t b) { return (b + 127) / 128 * 128; }
