@@ -163,7 +163,7 @@ int Batch::setup(int math, const bubble_batch_options *opt, std::string &err) {
     BATCH_CUDA(cudaMemsetAsync(d_scratch_, 0, scratch, stream_), "cudaMemset");
     d_counters_ = static_cast<unsigned int *>(d_scratch_);
     d_status_ = reinterpret_cast<int *>(static_cast<char *>(d_scratch_) + kOffStatus);
-    BATCH_CUDA(cudaMallocHost(reinterpret_cast<void **>(&h_result_), sizeof(DiagResult)), "cudaMallocHost");
+    BATCH_CUDA(cudaMallocHost(reinterpret_cast<void **>(&h_report_), sizeof(HostReport)), "cudaMallocHost");
     device_bytes_ += scratch;
     int maxg = launch::batch_max_grid(fast_, ty_);
     if (maxg <= 0) {
@@ -234,7 +234,7 @@ Batch::~Batch() {
     if (d_lat_) cudaFree(d_lat_);
     if (h_lat_) cudaFreeHost(h_lat_);
     if (d_scratch_) cudaFree(d_scratch_);
-    if (h_result_) cudaFreeHost(h_result_);
+    if (h_report_) cudaFreeHost(h_report_);
     if (stream_) cudaStreamDestroy(stream_);
 }
 
@@ -671,15 +671,15 @@ int Batch::diagnostics(uint32_t k, bubble_diag *out, std::string &err) {
     const size_t pb = (launch::diag_partials_bytes() + 255) & ~(size_t)255;
     char *base = static_cast<char *>(d_scratch_) + kOffDiag;
     unsigned int *ticket = reinterpret_cast<unsigned int *>(base + pb);
-    DiagResult *res = reinterpret_cast<DiagResult *>(base + pb + 256);
     BATCH_CUDA(launch::diag_f32((const V2<float> *)L.field[L.cur], (const V4<float> *)L.fluid[L.cur], L.P, false,
-                                base, ticket, res, stream_),
+                                base, ticket, &h_report_->result, d_status_, &h_report_->status, stream_),
                "diagnostics kernel");
-    BATCH_CUDA(cudaMemcpyAsync(h_result_, res, sizeof(DiagResult), cudaMemcpyDeviceToHost, stream_),
-               "diagnostics readback");
-    const int rc = check_status(err);
-    if (rc != BUBBLE_OK) return rc;
-    const DiagResult &r = *h_result_;
+    BATCH_CUDA(cudaStreamSynchronize(stream_), "cudaStreamSynchronize");
+    if (h_report_->status != 0) {
+        const int rc = check_status(err);
+        if (rc != BUBBLE_OK) return rc;
+    }
+    const DiagResult &r = h_report_->result;
     const float inv_n = 1.0f / (float)L.cells;
     bubble_diag d{};
     d.sum_energy = r.sums[0];

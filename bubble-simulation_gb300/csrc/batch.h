@@ -134,7 +134,7 @@ class Batch {
     unsigned int *d_counters_ = nullptr;
     int *d_status_ = nullptr;
     void *d_scratch_ = nullptr;  // counters | status | diag partials | ticket | result
-    DiagResult *h_result_ = nullptr;
+    HostReport *h_report_ = nullptr;  // pinned
     cudaStream_t stream_ = nullptr;
     uint64_t launches_ = 0;
     uint64_t device_bytes_ = 0;

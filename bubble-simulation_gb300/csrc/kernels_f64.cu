@@ -26,8 +26,8 @@ cudaError_t stage_ref_f64(const StageArgs<double> &A, const V4<double> *p,
 }
 cudaError_t diag_f64(const V2<double> *field, const V4<double> *fluid,
                      const LatticeParams<double> &P, void *partials, unsigned int *ticket,
-                     DiagResult *out, cudaStream_t s) {
-    return diag<double, false>(field, fluid, P, partials, ticket, out, s);
+                     DiagResult *out, const int *status, int *status_out, cudaStream_t s) {
+    return diag<double, false>(field, fluid, P, partials, ticket, out, s, status, status_out);
 }
 
 }  // namespace launch

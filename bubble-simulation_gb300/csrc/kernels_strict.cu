@@ -28,12 +28,13 @@ cudaError_t stage_ref_f32(const StageArgs<float> &A, const V4<float> *p,
 }
 cudaError_t diag_f32(const V2<float> *field, const V4<float> *fluid,
                      const LatticeParams<float> &P, int mode, void *partials,
-                     unsigned int *ticket, DiagResult *out, cudaStream_t s) {
-    if (mode == dev::kThermal) return diag<float, dev::kThermal>(field, fluid, P, partials, ticket, out, s);
-    if (mode == dev::kGamma) return diag<float, dev::kGamma>(field, fluid, P, partials, ticket, out, s);
-    if (mode == dev::kPert) return diag<float, dev::kPert>(field, fluid, P, partials, ticket, out, s);
-    if (mode == dev::kMixed) return diag<float, dev::kMixed>(field, fluid, P, partials, ticket, out, s);
-    return diag<float, dev::kPlain>(field, fluid, P, partials, ticket, out, s);
+                     unsigned int *ticket, DiagResult *out, const int *status, int *status_out,
+                     cudaStream_t s) {
+    if (mode == dev::kThermal) return diag<float, dev::kThermal>(field, fluid, P, partials, ticket, out, s, status, status_out);
+    if (mode == dev::kGamma) return diag<float, dev::kGamma>(field, fluid, P, partials, ticket, out, s, status, status_out);
+    if (mode == dev::kPert) return diag<float, dev::kPert>(field, fluid, P, partials, ticket, out, s, status, status_out);
+    if (mode == dev::kMixed) return diag<float, dev::kMixed>(field, fluid, P, partials, ticket, out, s, status, status_out);
+    return diag<float, dev::kPlain>(field, fluid, P, partials, ticket, out, s, status, status_out);
 }
 
 size_t diag_partials_bytes() { return sizeof(dev::DiagPartial) * dev::kDiagMaxBlocks; }

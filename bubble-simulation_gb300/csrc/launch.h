@@ -27,11 +27,13 @@ cudaError_t prim_f32(const V4<float> *fluid, V4<float> *prim, uint64_t n,
 cudaError_t stage_ref_f32(const StageArgs<float> &A, const V4<float> *prim,
                           const LatticeParams<float> &P, cudaStream_t s);
 
+// `out` and `status_out` (a copy of *status, or NULL) are written by the device
+// and may be pinned host memory.
 // `mode`: 0 plain, 1 mixed, 2 perturbation form, 3 gamma-law equation of
 // state, 4 thermal potential (physics.cuh kPlain/kMixed/kPert/kGamma/kThermal).
 cudaError_t diag_f32(const V2<float> *field, const V4<float> *fluid,
                      const LatticeParams<float> &P, int mode, void *partials,
-                     unsigned int *ticket, DiagResult *out, cudaStream_t s);
+                     unsigned int *ticket, DiagResult *out, const int *status, int *status_out, cudaStream_t s);
 
 // ---- FP64 (the FP64 CUDA oracle; no FMA contraction) --------------------
 cudaError_t init_f64(V2<double> *field, V4<double> *fluid, uint64_t n, double e_ref,
@@ -44,7 +46,7 @@ cudaError_t stage_ref_f64(const StageArgs<double> &A, const V4<double> *prim,
                           const LatticeParams<double> &P, cudaStream_t s);
 cudaError_t diag_f64(const V2<double> *field, const V4<double> *fluid,
                      const LatticeParams<double> &P, void *partials, unsigned int *ticket,
-                     DiagResult *out, cudaStream_t s);
+                     DiagResult *out, const int *status, int *status_out, cudaStream_t s);
 
 // Scratch of the diagnostics reduction: partials + ticket.
 size_t diag_partials_bytes();

@@ -171,13 +171,14 @@ cudaError_t stage_column16(const StageArgs<float> &A, const LatticeParams<float>
 
 template <typename R, int MIXED>
 cudaError_t diag(const V2<R> *field, const V4<R> *fluid, const LatticeParams<R> &P,
-                 void *partials, unsigned int *ticket, DiagResult *out, cudaStream_t s) {
+                 void *partials, unsigned int *ticket, DiagResult *out, cudaStream_t s, const int *status = nullptr,
+                 int *status_out = nullptr) {
     int device = 0, sms = 0;
     cudaGetDevice(&device);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
     const int blocks = dev::diag_blocks(P.nx, P.ny, P.nz, sms);
     return launch_dependent(dev::diag_kernel<R, MIXED>, dim3((unsigned)blocks), dev::kDiagThreads, 0, s, field, fluid, P,
-                            reinterpret_cast<dev::DiagPartial *>(partials), ticket, out);
+                            reinterpret_cast<dev::DiagPartial *>(partials), ticket, out, status, status_out);
 }
 
 }  // namespace launch_detail

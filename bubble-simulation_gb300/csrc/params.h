@@ -77,6 +77,13 @@ struct DiagResult {
     uint64_t cells;
 };
 
+// What a diagnostics launch leaves in pinned host memory: its result and the
+// status word of the bounded waits.
+struct HostReport {
+    DiagResult result;
+    int32_t status;
+};
+
 // Tile shape of the fused stage kernel.
 struct TileShape {
     int32_t tx, ty, lz;  // x, y tile (cells) and z chunk (planes)

@@ -196,7 +196,7 @@ int Simulation::create(const bubble_spec &spec, std::unique_ptr<Simulation> &out
 
 Simulation::~Simulation() {
     release();
-    if (h_result_) cudaFreeHost(h_result_);
+    if (h_report_) cudaFreeHost(h_report_);
     if (own_stream_ && stream_) cudaStreamDestroy(stream_);
 }
 
@@ -209,7 +209,6 @@ void Simulation::release() {
     for (int k = 0; k < 3; ++k) field_[k] = fluid_[k] = nullptr;
     partials_ = nullptr;
     ticket_ = nullptr;
-    d_result_ = nullptr;
     d_status_ = nullptr;
     tma_ok_ = false;
     device_bytes_ = 0;
@@ -244,7 +243,7 @@ int Simulation::allocate(std::string &err) {
         fluid_[k] = static_cast<char *>(state_) + k * slot + round_up(fb);
     }
     const size_t pb = round_up(launch::diag_partials_bytes());
-    const size_t scratch = pb + 256 + round_up(sizeof(DiagResult)) + 256;
+    const size_t scratch = pb + 256 + 256;
     e = device_alloc(&scratch_, scratch);
     if (e != cudaSuccess) {
         cudaGetLastError();
@@ -254,14 +253,13 @@ int Simulation::allocate(std::string &err) {
     }
     partials_ = scratch_;
     ticket_ = reinterpret_cast<unsigned int *>(static_cast<char *>(scratch_) + pb);
-    d_result_ = reinterpret_cast<DiagResult *>(static_cast<char *>(scratch_) + pb + 256);
-    d_status_ = reinterpret_cast<int *>(static_cast<char *>(scratch_) + pb + 256 + round_up(sizeof(DiagResult)));
+    d_status_ = reinterpret_cast<int *>(static_cast<char *>(scratch_) + pb + 256);
     BUBBLE_CUDA(cudaMemsetAsync(scratch_, 0, scratch, stream_), "cudaMemset");
     tma_ok_ = true;
     for (int k = 0; k < 3; ++k)
         tma_ok_ = tma_ok_ && encode_stage_maps(&maps_[k], field_[k], fluid_[k], (int)grid_[0], (int)grid_[1],
                                                (int)grid_[2], tile_.tx, tile_.ty, is_f64() ? 8 : 4);
-    if (!h_result_) BUBBLE_CUDA(cudaMallocHost(reinterpret_cast<void **>(&h_result_), sizeof(DiagResult)), "cudaMallocHost");
+    if (!h_report_) BUBBLE_CUDA(cudaMallocHost(reinterpret_cast<void **>(&h_report_), sizeof(HostReport)), "cudaMallocHost");
     device_bytes_ = 3 * slot + scratch;
     return BUBBLE_OK;
 }
@@ -614,22 +612,21 @@ int Simulation::diagnostics(bubble_diag *out, std::string &err) {
     cudaError_t e;
     if (is_f64()) {
         e = launch::diag_f64((const V2<double> *)field_[cur_], (const V4<double> *)fluid_[cur_],
-                             params_f64(), partials_, ticket_, d_result_, stream_);
+                             params_f64(), partials_, ticket_, &h_report_->result, d_status_, &h_report_->status,
+                             stream_);
     } else {
         e = launch::diag_f32((const V2<float> *)field_[cur_], (const V4<float> *)fluid_[cur_],
-                             params_f32(), arith_mode(), partials_,
-                             ticket_, d_result_, stream_);
+                             params_f32(), arith_mode(), partials_, ticket_, &h_report_->result, d_status_,
+                             &h_report_->status, stream_);
     }
     ++launches_;
     BUBBLE_CUDA(e, "diagnostics kernel");
-    BUBBLE_CUDA(cudaMemcpyAsync(h_result_, d_result_, sizeof(DiagResult), cudaMemcpyDeviceToHost, stream_),
-                "diagnostics readback");
     BUBBLE_CUDA(cudaStreamSynchronize(stream_), "cudaStreamSynchronize");
-    {
+    if (h_report_->status != 0) {
         const int rc = check_status(err);
         if (rc != BUBBLE_OK) return rc;
     }
-    DiagResult r = *h_result_;
+    DiagResult r = h_report_->result;
     if (spec_.precision == BUBBLE_PRECISION_PERTURBATION) {
         // the kernel summed E - e_bg: add the background in FP64
         const double bg = (double)params_f32().e_bg * (double)n_cells_;

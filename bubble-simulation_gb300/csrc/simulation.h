@@ -137,9 +137,8 @@ class Simulation {
     void *scratch_ = nullptr;   // diag partials | ticket | result | status
     void *partials_ = nullptr;
     unsigned int *ticket_ = nullptr;
-    DiagResult *d_result_ = nullptr;
     int *d_status_ = nullptr;   // bit 0: a bounded wait in a stage kernel expired
-    DiagResult *h_result_ = nullptr;  // pinned
+    HostReport *h_report_ = nullptr;  // pinned
     uint64_t device_bytes_ = 0;
     StageMaps maps_[3];         // TMA maps of each slot as a stage input
     bool tma_ok_ = false;
