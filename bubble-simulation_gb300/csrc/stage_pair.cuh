@@ -17,18 +17,22 @@
 //
 // What bounds it.  The scalar column form issued 26.6 warp instructions per
 // cell and stage (256^3, MIXED) and was bound by that; the pair form issues
-// 15.9.  Packed FP32 takes the FMA pipe as long as two scalar instructions
+// 16.2 (15.5 in the first stage).  Packed FP32 takes the FMA pipe as long as two scalar instructions
 // (0.36 fma.f32x2 and 0.49 add.f32x2 or mul.f32x2 per clock and scheduler,
 // measured, against 0.61 fma and 0.93 add), so it saves issue slots, not
-// arithmetic time: FMA pipe 52 %, shared-memory data path 64 %, issue 58 % at
+// arithmetic time: FMA pipe 50 %, shared-memory data path 63 %, issue 59 % at
 // 14 warps per SM, the rest dependency latency and barriers.  Registers set
 // the residency: 15 warps over four schedulers leave 128 per thread.  Measured
 // and not kept: 16 warps in four CTAs without a halo warp (equal on large
 // lattices, slower below 160^3), the axes on separate warps at 72 registers
 // (barrier-bound), U_in and U^n loaded at the combine (8 % slower), the march
-// unrolled by 2 or 3 (20 to 30 % slower).  Step time, column form to pair
-// form (GB300): 512^3 MIXED 10.85 -> 8.18 ms, 256^3 perturbation 1.54 -> 1.16
-// ms, 128^3 0.212 -> 0.170 ms, 64^3 49.3 -> 43.1 us; the gamma law at 128^3,
+// unrolled by 2 or 3 (20 to 30 % slower), the plane barriers split into
+// mbarrier arrivals and waits around independent work (1 to 4 % slower), the
+// first stage in its own instantiation (1 % faster from 128^3, 1 % slower at
+// 64^3 and below, where two kernels alternate).  Step time, column form to
+// pair form (GB300): 512^3 MIXED 10.85 -> 8.25 ms, 256^3 perturbation 1.54 ->
+// 1.16 ms, 128^3 0.212 -> 0.170 ms, 64^3 49.3 -> 43.1 us (0.160 ms and 36.5 us
+// with dependent launches and the form's own z chunk); the gamma law at 128^3,
 // with its recovery in closed form, 0.33 -> 0.18 ms, the thermal potential at
 // 96^3, with its short iterations, 0.374 -> 0.177 ms (0.240 at two CTAs per SM,
 // where it has no spills).
@@ -112,14 +116,15 @@ BUBBLE_DEV void put_half(float4 *a, int c, const P4 &q) {
 // The last stage rounds u1 on its own: U^n + a1 (dt L + (U_in - U^n)), with
 // one rounding less, drops every increment below 3/4 ulp where rounding u1
 // drops those below 1/2, and left twice the error in E and Z after 100 steps of
-// 128^3.  The mixed form, whose cells with gamma > 3 magnify the rounding of E
-// and Z, takes the order with one rounding less in the middle stage: largest
-// errors 0.69 .. 0.80 of the strict form's against 0.73 .. 0.82 (random
-// relativistic states), 512^3 8.16 -> 8.22 ms.
+// 128^3.  Cells of the mixed form beyond gamma = 3 (om = 1 - v^2 below 1/9),
+// which magnify the rounding of E and Z, take the order with one rounding
+// less in the middle stage: there it lowers the largest errors, and in every
+// cell it would raise the energy's drift over 3000 steps (256^3: 6.8e-8 of it
+// beyond FP64's, 8.9e-8 with every cell).  512^3 8.16 -> 8.25 ms.
 template <int FORM>
 BUBBLE_DEV void store_cell(const StageArgs<float> &A, uint32_t g, const V2<float> &pf, const V4<float> &pu,
                            const V2<float> &pfn, const V4<float> &pun, float d_pi, float d_e, float d_x, float d_y,
-                           float d_z) {
+                           float d_z, float om) {
     const float dt = A.dt;
     if (A.stage == 0) {
         A.field_out[g] = V2<float>{__fmaf_rn(dt, pf.y, pf.x), __fmaf_rn(dt, d_pi, pf.y)};
@@ -129,7 +134,7 @@ BUBBLE_DEV void store_cell(const StageArgs<float> &A, uint32_t g, const V2<float
         const float a1 = A.a1;
         auto comb = [&](float d, float u, float n) { return __fmaf_rn(a1, __fsub_rn(__fmaf_rn(dt, d, u), n), n); };
         A.field_out[g] = V2<float>{comb(pf.y, pf.x, pfn.x), comb(d_pi, pf.y, pfn.y)};
-        const bool mid = FORM == kMixed && A.stage == 1;
+        const bool mid = FORM == kMixed && A.stage == 1 && om < 1.0f / 9.0f;
         auto comb_u = [&](float d, float u, float n) {
             const float two = __fsub_rn(__fmaf_rn(dt, d, u), n), one = __fmaf_rn(dt, d, __fsub_rn(u, n));
             return __fmaf_rn(a1, mid ? one : two, n);
@@ -412,8 +417,8 @@ BUBBLE_DEV bool pair_item(unsigned char *smem, const StageArgs<float> &A, const 
                 const float2 d_x = p_fma(nd, gx, div(xl.y, xu.y, yl.y, yu.y, fz_m.y, fz_p.y));
                 const float2 d_y = p_fma(nd, gy, div(xl.z, xu.z, yl.z, yu.z, fz_m.z, fz_p.z));
                 const float2 d_z = p_fma(nd, gz, div(xl.w, xu.w, yl.w, yu.w, fz_m.w, fz_p.w));
-                if (v0) store_cell<FORM>(A, base + g0, pf0, pu0, pn0, un0, d_pi.x, d_e.x, d_x.x, d_y.x, d_z.x);
-                if (v1) store_cell<FORM>(A, base + g1, pf1, pu1, pn1, un1, d_pi.y, d_e.y, d_x.y, d_y.y, d_z.y);
+                if (v0) store_cell<FORM>(A, base + g0, pf0, pu0, pn0, un0, d_pi.x, d_e.x, d_x.x, d_y.x, d_z.x, om.x);
+                if (v1) store_cell<FORM>(A, base + g1, pf1, pu1, pn1, un1, d_pi.y, d_e.y, d_x.y, d_y.y, d_z.y, om.y);
             }
             q0 = q1;
             q1 = q2;
