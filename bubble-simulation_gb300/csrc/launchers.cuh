@@ -141,9 +141,9 @@ cudaError_t stage_pair(const StageArgs<float> &A, const LatticeParams<float> &P,
 
 // Whether a 16 x 16 FP32 launch of the column kernel takes the shared form: on request, or
 // (BUBBLE_STAGE_FORM_AUTO) when column_stage_cost (params.h) rates it cheaper
-// at this chunk.  Measured per step, register vs shared form: 128^3 (256
-// CTAs) 0.239 vs 0.261 ms, 256^3 (2048 CTAs) 1.549 vs 1.508 ms, 512^3 (4096
-// CTAs) 11.38 vs 11.03 ms.
+// at this chunk.  Measured per step (strict arithmetic, the form's default
+// chunk), register vs shared form: 64^3 0.071 vs 0.068 ms, 128^3 0.597 vs 0.482
+// ms, 256^3 4.71 vs 4.13 ms, 512^3 36.1 vs 31.3 ms.
 inline bool shared_form(const LatticeParams<float> &P, const TileShape &shape) {
     if (shape.form == BUBBLE_STAGE_FORM_SHARED) return true;
     if (shape.form == BUBBLE_STAGE_FORM_REGISTERS) return false;
