@@ -7,9 +7,10 @@
 // The formulas are those of the shaders cited in physics.cuh; every rounding
 // is explicit, so each call site computes the same bits.
 //
-// The rarely needed parts -- primitive recovery above gamma = 3 (with the
-// FP64 recovery of the MIXED and perturbation forms and the |Z| cap) and the
-// velocity clamp of a face state -- are decided by one test per pair.
+// The rarely needed parts -- primitive recovery above gamma = 3 or at the
+// pressure floor (with the FP64 recovery of the MIXED and perturbation forms
+// and the |Z| cap) and the velocity clamp of a face state -- are decided by one
+// test per pair.
 #pragma once
 
 #include "physics.cuh"
@@ -37,6 +38,12 @@ BUBBLE_DEV float2 dot3_2(float2 x, float2 y, float2 z) { return p_fma(z, z, p_fm
 BUBBLE_DEV float min_xorsign(float a, float b) {
     float r;
     asm("min.xorsign.abs.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
+    return r;
+}
+// the smaller of both, NaN if either is
+BUBBLE_DEV float min_nan(float a, float b) {
+    float r;
+    asm("min.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
     return r;
 }
 
@@ -165,10 +172,12 @@ static __device__ __noinline__ V4<float> recover_slow_thermal(V4<float> u, float
 
 // sanitise(recover(u)) of two cells in two parts, so independent work can be
 // scheduled between them: recover_pair evaluates both cells by the formulas
-// that hold below gamma = 3; recover_fix sends a cell whose |v|^2 came out
-// above 8/9 (gamma > 3) through the scalar recovery.  That covers every cell
-// whose |Z| exceeds z_max E: the cap leaves |v|^2 > 8/9, and without it the
-// result is larger still (p is floored when E^2 - Z^2 is not positive).
+// that hold below gamma = 3 and above the pressure floor, which it does not
+// apply; recover_fix sends a cell whose |v|^2 came out above 8/9 (gamma > 3)
+// or whose p is below the floor or NaN through the scalar recovery.  Together
+// they cover every cell whose |Z| exceeds z_max E: the uncapped p of the bag
+// forms and the gamma law is then below the floor, NaN, or so small that |v|^2
+// is above 8/9 (where the floor is comparable to E, |v| alone can stay below).
 template <int FORM>
 BUBBLE_DEV P4 recover_pair(const V4<float> &ua, const V4<float> &ub, float2 phi, const LatticeParams<float> &P) {
     const float2 de = max2(make_float2(ua.x, ub.x), P.e_floor);
@@ -178,12 +187,12 @@ BUBBLE_DEV P4 recover_pair(const V4<float> &ua, const V4<float> &ub, float2 phi,
         // with s = E + p the closure is s^2 - B s + c2 Z^2 = 0, B = E + c2 (E -
         // e0), whose larger root the Newton steps of prim_from_cons_gamma
         // approach; p = c2 (E - e0 - Z^2 / s) keeps p's digits.  No real root
-        // (NaN) and a root below the floor both end at the floor.
+        // (NaN) and a root below the floor both go through recover_fix.
         const float2 x = p_sub(de, bc2(P.eos_e0));
         const float2 b = p_fma(bc2(P.eos_c2), x, de);
         const float2 sq = sqrt2(p_fma(b, b, p_mul(bc2(-4.0f * P.eos_c2), z2)));
         const float2 s = p_mul(bc2(0.5f), p_add(b, sq));
-        const float2 p = max2(p_mul(bc2(P.eos_c2), p_sub(x, p_mul(z2, rcp2(s)))), P.p_floor);
+        const float2 p = p_mul(bc2(P.eos_c2), p_sub(x, p_mul(z2, rcp2(s))));
         const float2 inv = rcp2(p_add(de, p));
         return P4{p_mul(zx, inv), p_mul(zy, inv), p_mul(zz, inv), p};
     }
@@ -226,10 +235,10 @@ BUBBLE_DEV P4 recover_pair(const V4<float> &ua, const V4<float> &ub, float2 phi,
     float2 p, s;
     if constexpr (FORM == kPert) {
         const float2 t = p_mul(z2, rcp2(p_fma(bc2(2.0f), e, sq)));
-        p = max2(p_fma(de, bc2((float)(1.0 / 3.0)), p_mul(t, bc2(-1.0f))), P.p_floor);
+        p = p_fma(de, bc2((float)(1.0 / 3.0)), p_mul(t, bc2(-1.0f)));
         s = p_add(p_add(e, bc2(P.p_bg)), p);
     } else {
-        p = max2(p_mul(p_fma(e, e, p_mul(z2, bc2(-1.0f))), rcp2(p_add(e, sq))), P.p_floor);
+        p = p_mul(p_fma(e, e, p_mul(z2, bc2(-1.0f))), rcp2(p_add(e, sq)));
         s = p_add(e, p);
     }
     const float2 inv = rcp2(s);
@@ -240,7 +249,7 @@ BUBBLE_DEV void recover_fix(P4 &q, const V4<float> *ua, const V4<float> *ub, flo
                             const LatticeParams<float> &P) {
     const float2 v2 = dot3_2(q.x, q.y, q.z);
     constexpr float kFast = 8.0f / 9.0f;
-    if (fmaxf(v2.x, v2.y) > kFast) {
+    if (fmaxf(v2.x, v2.y) > kFast || !(min_nan(q.w.x, q.w.y) >= P.p_floor)) {
         auto slow = [&](const V4<float> *u, float f) {
             if constexpr (FORM == kThermal)
                 return recover_slow_thermal(*u, f, P.e_floor, P.z_max, P.p_floor, P.th_k, P.th_g, P.th_h, P.th_i2a,
@@ -249,14 +258,14 @@ BUBBLE_DEV void recover_fix(P4 &q, const V4<float> *ua, const V4<float> *ub, flo
                 return recover_slow<FORM>(*u, P.e_floor, P.z_max, P.p_floor, FORM == kGamma ? P.eos_c2 : P.e_bg,
                                           FORM == kGamma ? P.eos_e0 : P.p_bg);
         };
-        if (v2.x > kFast) {
+        if (v2.x > kFast || !(q.w.x >= P.p_floor)) {
             const V4<float> r = slow(ua, phi.x);
             q.x.x = r.x;
             q.y.x = r.y;
             q.z.x = r.z;
             q.w.x = r.w;
         }
-        if (v2.y > kFast) {
+        if (v2.y > kFast || !(q.w.y >= P.p_floor)) {
             const V4<float> r = slow(ub, phi.y);
             q.x.y = r.x;
             q.y.y = r.y;
