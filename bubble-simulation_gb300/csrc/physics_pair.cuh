@@ -187,11 +187,14 @@ BUBBLE_DEV P4 recover_pair(const V4<float> &ua, const V4<float> &ub, float2 phi,
         // with s = E + p the closure is s^2 - B s + c2 Z^2 = 0, B = E + c2 (E -
         // e0), whose larger root the Newton steps of prim_from_cons_gamma
         // approach; p = c2 (E - e0 - Z^2 / s) keeps p's digits.  No real root
-        // (NaN) and a root below the floor both go through recover_fix.
+        // (NaN) and a p below the floor both go through recover_fix.  For B <= 0
+        // the root is all cancellation, a few units of B's last place of either
+        // sign; held at 0 it gives p = -inf or NaN, and a positive one gives p
+        // below c2 (E - e0) < 0.
         const float2 x = p_sub(de, bc2(P.eos_e0));
         const float2 b = p_fma(bc2(P.eos_c2), x, de);
         const float2 sq = sqrt2(p_fma(b, b, p_mul(bc2(-4.0f * P.eos_c2), z2)));
-        const float2 s = p_mul(bc2(0.5f), p_add(b, sq));
+        const float2 s = max2(p_mul(bc2(0.5f), p_add(b, sq)), 0.0f);
         const float2 p = p_mul(bc2(P.eos_c2), p_sub(x, p_mul(z2, rcp2(s))));
         const float2 inv = rcp2(p_add(de, p));
         return P4{p_mul(zx, inv), p_mul(zy, inv), p_mul(zz, inv), p};

@@ -62,3 +62,29 @@ def test_momentum_beyond_the_cap_at_the_energy_floor(bubble, gpu, precision, eos
     r = np.random.default_rng(1).choice([1.01, 1.2, 1.5, 1.85, 2.0], size=len(e))
     f0, u0 = _state(e, DIRECTION * (r * e)[:, None])
     _compare(bubble, GRID, f0, u0, precision, eos, eos_param)
+
+
+@pytest.mark.parametrize("gamma,e0", [(1.2, 0.05), (2.0, 0.12), (1.02, 0.12)])
+def test_gamma_law_energy_below_its_offset(bubble, gpu, gamma, e0):
+    """For E below e0 c2 / (1 + c2) the quadratic of the closed form has only
+    roots that are rounding errors; the pressure is the floor.  Read through
+    the friction of a uniform lattice, d pi / dt = -eta W(v) pi with v = Z /
+    (E + p), where nothing else acts: the flux of such a state is of the order
+    of e0, and its rounding would cover Z.  |v| <= 0.9, so dW / dv <= 11 and
+    the bar of 1e-5 is a hundred roundings of v."""
+    grid, pi = (8, 8, 8), 1e-6
+    n = grid[0] * grid[1] * grid[2]
+    spec = bubble.SimulationSpec(grid=grid, bubbles=0, nucleation="centre", eos="gamma_law", eos_param=(gamma, e0))
+    got = {}
+    for math in ("strict", "fast"):
+        spec.math = math
+        got[math] = []
+        with bubble.Simulation(spec) as sim:
+            for e in np.geomspace(1e-6, 1e-3, 41):
+                for r in (0.01, 0.3, 0.6, 0.75, 0.9):
+                    e32 = np.full(n, e, np.float32)
+                    sim.load_state(*_state(e32, np.outer(r * e32, DIRECTION), pi=pi))
+                    sim.advance(1)
+                    got[math].append(sim.copy_state()[0][:, 1].astype(np.float64) / pi)
+    err = np.max(np.abs(np.array(got["fast"]) - np.array(got["strict"])), axis=1)
+    assert np.all(err <= 1e-5), (np.flatnonzero(err > 1e-5), err.max())
