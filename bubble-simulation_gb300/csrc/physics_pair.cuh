@@ -177,7 +177,8 @@ static __device__ __noinline__ V4<float> recover_slow_thermal(V4<float> u, float
 // or whose p is below the floor or NaN through the scalar recovery.  Together
 // they cover every cell whose |Z| exceeds z_max E: the uncapped p of the bag
 // forms and the gamma law is then below the floor, NaN, or so small that |v|^2
-// is above 8/9 (where the floor is comparable to E, |v| alone can stay below).
+// is above 8/9 (where the floor is comparable to E, |v| alone can stay below);
+// the thermal potential tests |Z| itself.
 template <int FORM>
 BUBBLE_DEV P4 recover_pair(const V4<float> &ua, const V4<float> &ub, float2 phi, const LatticeParams<float> &P) {
     const float2 de = max2(make_float2(ua.x, ub.x), P.e_floor);
@@ -201,8 +202,9 @@ BUBBLE_DEV P4 recover_pair(const V4<float> &ua, const V4<float> &ub, float2 phi,
     }
     if constexpr (FORM == kThermal) {
         // Newton on f(p) = p - p(T(e), phi) from the Z = 0 root, e = E - Z^2 / (E
-        // + p): three steps; a cell whose last step is above 2e-4 p gets v out
-        // of range, which sends it to recover_fix
+        // + p): three steps; a cell whose last step is above 2e-4 p, or whose |Z|
+        // is beyond the cap (cold cells have p > e there and |v| below the
+        // threshold), gets v out of range, which sends it to recover_fix
         const ThermalPair f = thermal_pair(phi, P);
         const float2 a4 = bc2(4.0f * P.a_rad), b2 = p_mul(f.b, f.b);
         float2 p, dp = make_float2(0.0f, 0.0f), e = de, isp = dp;
@@ -229,8 +231,9 @@ BUBBLE_DEV P4 recover_pair(const V4<float> &ua, const V4<float> &ub, float2 phi,
         }
         const float2 inv = rcp2(p_add(de, p));
         P4 q{p_mul(zx, inv), p_mul(zy, inv), p_mul(zz, inv), p};
-        if (!(fabsf(dp.x) <= 2e-4f * p.x)) q.x.x = 2.0f;
-        if (!(fabsf(dp.y) <= 2e-4f * p.y)) q.x.y = 2.0f;
+        const float2 over = p_fma(p_mul(bc2(-P.z_max * P.z_max), de), de, z2);
+        if (!(fabsf(dp.x) <= 2e-4f * p.x && over.x <= 0.0f)) q.x.x = 2.0f;
+        if (!(fabsf(dp.y) <= 2e-4f * p.y && over.y <= 0.0f)) q.x.y = 2.0f;
         return q;
     }
     const float2 e = FORM == kPert ? p_add(bc2(P.e_bg), de) : de;
@@ -252,7 +255,8 @@ BUBBLE_DEV void recover_fix(P4 &q, const V4<float> *ua, const V4<float> *ub, flo
                             const LatticeParams<float> &P) {
     const float2 v2 = dot3_2(q.x, q.y, q.z);
     constexpr float kFast = 8.0f / 9.0f;
-    if (fmaxf(v2.x, v2.y) > kFast || !(min_nan(q.w.x, q.w.y) >= P.p_floor)) {
+    // (the thermal form floors p and marks the cells itself)
+    if (fmaxf(v2.x, v2.y) > kFast || (FORM != kThermal && !(min_nan(q.w.x, q.w.y) >= P.p_floor))) {
         auto slow = [&](const V4<float> *u, float f) {
             if constexpr (FORM == kThermal)
                 return recover_slow_thermal(*u, f, P.e_floor, P.z_max, P.p_floor, P.th_k, P.th_g, P.th_h, P.th_i2a,

@@ -88,3 +88,66 @@ def test_gamma_law_energy_below_its_offset(bubble, gpu, gamma, e0):
                     got[math].append(sim.copy_state()[0][:, 1].astype(np.float64) / pi)
     err = np.max(np.abs(np.array(got["fast"]) - np.array(got["strict"])), axis=1)
     assert np.all(err <= 1e-5), (np.flatnonzero(err > 1e-5), err.max())
+
+
+THERMAL = [(0.0125, 0.05), (0.999 * 0.125 / 6.0, 0.999 * 0.125 / np.sqrt(2.0))]
+
+
+def _thermal_energy(gamma, T, phi):
+    return 0.125 * T**4 - 0.5 * gamma * (T * phi) ** 2
+
+
+def _pi_after_a_step(bubble, states, eos_param, pi):
+    """pi of uniform lattices (e, |Z|, phi) after one step, strict and fast."""
+    grid, n = (8, 8, 8), 512
+    spec = bubble.SimulationSpec(grid=grid, bubbles=0, nucleation="centre", eos="thermal", eos_param=eos_param)
+    got = {}
+    for math in ("strict", "fast"):
+        spec.math = math
+        got[math] = []
+        with bubble.Simulation(spec) as sim:
+            for e, z, phi in states:
+                sim.load_state(*_state(np.full(n, e), np.outer(np.full(n, z), DIRECTION), phi=phi, pi=pi))
+                sim.advance(1)
+                got[math].append(sim.copy_state()[0][:, 1].astype(np.float64))
+    return np.array(got["strict"]), np.array(got["fast"])
+
+
+def _thermal_speed(eos_param, e, z, phi):
+    """|v| of a cell in 64 bits, |Z| capped at 0.9999 E: bisection on the pressure."""
+    gamma, a = eos_param
+    z = min(z, 0.9999 * e)
+
+    def excess(p):
+        b, en = gamma * phi**2, e - z * z / (e + p)
+        T = np.sqrt((0.5 * b + np.sqrt(0.25 * b * b + 0.5 * en)) / 0.25)
+        return p - (0.125 / 3.0 * T**4 - 0.5 * b * T * T + a / 3.0 * T * phi**3)
+
+    lo, hi = 0.0, 10.0
+    for _ in range(200):
+        mid = 0.5 * (lo + hi)
+        lo, hi = (mid, hi) if excess(mid) < 0.0 else (lo, mid)
+    return z / (e + lo)
+
+
+@pytest.mark.parametrize("eos_param", THERMAL)
+def test_thermal_momentum_beyond_the_cap(bubble, gpu, eos_param):
+    """Cold cells of the thermal potential have p > e, so |v| stays below the
+    gamma = 3 threshold for |Z| beyond the cap.  Read through pi of uniform
+    lattices, on which friction (W of v) and the thermal force (T) act and no
+    flux.  Lattices of |v| < 0.8 when capped: the bar is then a hundred
+    roundings of v (dW / dv <= 4; at W = 70, which capped warm cells reach, one
+    rounding of v alone is 2e-2 of W)."""
+    gamma, _ = eos_param
+    branch = np.sqrt(3.0 * gamma / 0.5)
+    states = []
+    for T in (0.2, 0.26, 0.35, 0.5, 0.7, 1.0):
+        for phi in (0.0, 0.3, 0.71, 1.0):
+            if T >= 1.02 * branch * phi:
+                e = _thermal_energy(gamma, T, phi)
+                states += [(e, r * e, phi) for r in (0.0, 0.5, 0.9, 1.1, 1.27, 1.6)
+                           if _thermal_speed(eos_param, e, r * e, phi) < 0.8]
+    assert sum(z > e for e, z, _ in states) >= 3  # some beyond the cap
+    strict, fast = _pi_after_a_step(bubble, states, eos_param, pi=0.01)
+    err = np.max(np.abs(fast - strict), axis=1) / np.max(np.abs(strict), axis=1)
+    assert np.all(err <= 1e-5), [(states[k], err[k]) for k in np.flatnonzero(err > 1e-5)]
