@@ -108,22 +108,25 @@ BUBBLE_DEV float2 thermal_step(float2 &t, float2 p, const ThermalPair &f, const 
 // eos_temperature(p, phi).  Newton's steps converge quadratically from the phi
 // = 0 root: where the first is below 1e-4 T its successor is below rounding
 // (all of the symmetric phase); otherwise three more follow, and a cell whose
-// last step is still above 2e-4 T, or that left the branch T >= lo |phi|, takes
-// the bounded iteration.  Values accepted early are within 7.4e-8 T of the
-// root (64-bit evaluation over T >= 0.4 T_ref, -0.3 <= phi/phi_b <= 1.2 and the
-// validated gamma and A).  Each half is decided on its own values, so a pair's
-// halves do not affect each other.
+// last step is still above 2e-4 T takes the bounded iteration.  So does a cell
+// that left the branch T >= lo |phi|: for A below 1.5 gamma lo the phi = 0 root can
+// itself solve p(T, phi) = p off the branch, at T = 2 A phi / (3 gamma).  Values
+// accepted early are within 1.1e-7 T of the root, later ones within 2.2e-7, as
+// the bounded iteration's are (FP32 rounding against 64 bits, T from the branch
+// limit to 1.3 T_ref, -0.3 <= phi/phi_b <= 1.2 and the validated gamma and A).
+// Each half is decided on its own values, so a pair's halves do not affect each
+// other.
 BUBBLE_DEV float2 temperature_pair(float2 p, const ThermalPair &f, const LatticeParams<float> &P) {
     const float2 t0 = sqrt2(sqrt2(p_mul(p, bc2(P.th_ik))));
     float2 t1 = t0;
     const float2 d1 = thermal_step(t1, p, f, P);
-    const bool cx = fabsf(d1.x) <= 1e-4f * t1.x, cy = fabsf(d1.y) <= 1e-4f * t1.y;
+    const float lx = P.th_lo * fabsf(f.phi.x), ly = P.th_lo * fabsf(f.phi.y);
+    const bool cx = fabsf(d1.x) <= 1e-4f * t1.x && t1.x >= lx, cy = fabsf(d1.y) <= 1e-4f * t1.y && t1.y >= ly;
     if (cx && cy) return t1;
     float2 t = t1;
     thermal_step(t, p, f, P);
     thermal_step(t, p, f, P);
     const float2 d = thermal_step(t, p, f, P);
-    const float lx = P.th_lo * fabsf(f.phi.x), ly = P.th_lo * fabsf(f.phi.y);
     if (!cx && !(fabsf(d.x) <= 2e-4f * t.x && t.x >= lx))
         t.x = temperature_slow(p.x, f.phi.x, P.th_k, P.th_g, P.th_h, P.th_lo, P.p_floor);
     if (!cy && !(fabsf(d.y) <= 2e-4f * t.y && t.y >= ly))

@@ -151,3 +151,18 @@ def test_thermal_momentum_beyond_the_cap(bubble, gpu, eos_param):
     strict, fast = _pi_after_a_step(bubble, states, eos_param, pi=0.01)
     err = np.max(np.abs(fast - strict), axis=1) / np.max(np.abs(strict), axis=1)
     assert np.all(err <= 1e-5), [(states[k], err[k]) for k in np.flatnonzero(err > 1e-5)]
+
+
+@pytest.mark.parametrize("phi", [0.4, 1.0, 1.2])
+def test_thermal_temperature_off_the_branch(bubble, gpu, phi):
+    """With A < 1.5 gamma lo the phi = 0 root of the pressure solves p(T, phi) = p
+    at T* = 2 A phi / (3 gamma), off the branch T >= lo phi, where the inversion
+    must not stop.  Lattices at rest whose recovered T is T* within 3e-4; pi
+    after a step is the thermal force at the inverted T."""
+    gamma, a = 0.0208, 0.0095
+    t_star = 2.0 * a * phi / (3.0 * gamma)
+    assert np.sqrt(gamma / 0.25) * phi < t_star < np.sqrt(3.0 * gamma / 0.5) * phi
+    states = [(_thermal_energy(gamma, t_star * (1.0 + d), phi), 0.0, phi) for d in np.linspace(-3e-4, 3e-4, 61)]
+    strict, fast = _pi_after_a_step(bubble, states, (gamma, a), pi=0.0)
+    err = np.max(np.abs(fast - strict), axis=1) / np.max(np.abs(strict), axis=1)
+    assert np.all(err <= 1e-5), [(states[k], err[k]) for k in np.flatnonzero(err > 1e-5)]
