@@ -109,19 +109,25 @@ BUBBLE_DEV float2 thermal_step(float2 &t, float2 p, const ThermalPair &f, const 
 // = 0 root: where the first is below 1e-4 T its successor is below rounding
 // (all of the symmetric phase); otherwise three more follow, and a cell whose
 // last step is still above 2e-4 T takes the bounded iteration.  So does a cell
-// that left the branch T >= lo |phi|: for A below 1.5 gamma lo the phi = 0 root can
-// itself solve p(T, phi) = p off the branch, at T = 2 A phi / (3 gamma).  Values
-// accepted early are within 1.1e-7 T of the root, later ones within 2.2e-7, as
-// the bounded iteration's are (FP32 rounding against 64 bits, T from the branch
-// limit to 1.3 T_ref, -0.3 <= phi/phi_b <= 1.2 and the validated gamma and A).
-// Each half is decided on its own values, so a pair's halves do not affect each
-// other.
+// that left the branch T >= lo |phi|.  The early step can end off it only for A
+// below 1.5 gamma lo, where the phi = 0 root itself solves p(T, phi) = p at T = 2
+// A phi / (3 gamma) < lo phi (for A >= 1.6 gamma lo a first step from off the
+// branch is above 2e-2 T); only there is it tested (96^3 step 177.7 us, 181
+// tested always).  Values accepted early are within 1.1e-7 T of the root, later
+// ones within 2.2e-7, as the bounded iteration's are (FP32 rounding against 64
+// bits, T from the branch limit to 1.3 T_ref, -0.3 <= phi/phi_b <= 1.2 and the
+// validated gamma and A).  Each half is decided on its own values, so a pair's
+// halves do not affect each other.
 BUBBLE_DEV float2 temperature_pair(float2 p, const ThermalPair &f, const LatticeParams<float> &P) {
     const float2 t0 = sqrt2(sqrt2(p_mul(p, bc2(P.th_ik))));
     float2 t1 = t0;
     const float2 d1 = thermal_step(t1, p, f, P);
     const float lx = P.th_lo * fabsf(f.phi.x), ly = P.th_lo * fabsf(f.phi.y);
-    const bool cx = fabsf(d1.x) <= 1e-4f * t1.x && t1.x >= lx, cy = fabsf(d1.y) <= 1e-4f * t1.y && t1.y >= ly;
+    bool cx = fabsf(d1.x) <= 1e-4f * t1.x, cy = fabsf(d1.y) <= 1e-4f * t1.y;
+    if (P.th_a < 1.6f * P.th_g * P.th_lo) {
+        cx = cx && t1.x >= lx;
+        cy = cy && t1.y >= ly;
+    }
     if (cx && cy) return t1;
     float2 t = t1;
     thermal_step(t, p, f, P);
