@@ -14,6 +14,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <type_traits>
+
 #include "params.h"
 #include "physics.cuh"
 
@@ -269,7 +271,9 @@ __global__ void stage_ref_kernel(StageArgs<R> A, const V4<R> *__restrict__ prim,
 // is a sum of at most 32 terms below 2^-24 hi, so a chunk's pair is within
 // 2^-44 of exact, unbiased, and the total over many chunks well below that
 // (the fluid energies of 64^3 to 256^3 states sum to the correctly rounded
-// double).  The largest speed is taken from the largest |v|^2 (sqrt is
+// double).  A chunk whose sums leave the FP32 range (terms above 1e37,
+// infinities, NaN) is marched again with each term added in FP64 (in code of its
+// own: 512^3 1.34 -> 1.37 ms; a flag in the loop: 1.48).  The largest speed is taken from the largest |v|^2 (sqrt is
 // monotone).  Now 1.27 ms at 512^3, bound by instruction issue; 256^3 0.59 ->
 // 0.21 ms, 128^3 96 -> 60 us.
 constexpr int kDiagThreads = 256;
@@ -312,11 +316,6 @@ struct TermSum {
         } else {
             hi += x;
         }
-    }
-    BUBBLE_DEV double take() {
-        const double v = (double)hi + (double)lo;
-        hi = lo = R(0);
-        return v;
     }
 };
 
@@ -394,57 +393,73 @@ __global__ void __launch_bounds__(kDiagThreads, kDiagBlocksPerSm)
         const uint32_t cxp = x + 1 < P.nx ? c + 1 : c + 1 - P.nx, cxm = x > 0 ? c - 1 : c - 1 + P.nx;
         const uint32_t cyp = y + 1 < P.ny ? c + P.nx : c + P.nx - plane, cym = y > 0 ? c - P.nx : c - P.nx + plane;
         const int z0 = (int)chunk * lz, z1 = min(z0 + lz, P.nz);
-        // cell indices fit 32 bits
-        R phi_m = field[(uint32_t)wrap1(z0 - 1, P.nz) * plane + c].x;
-        V2<R> f = field[(uint32_t)z0 * plane + c];
         TermSum<R> s_total, s_kinetic, s_e;
-        uint32_t broken = 0;
+        // The chunk's terms into the pairs, or (WIDE) each into the FP64 sums;
+        // returns its cells in the broken phase.
+        auto march = [&](auto wide) {
+            constexpr bool WIDE = decltype(wide)::value;
+            // cell indices fit 32 bits
+            R phi_m = field[(uint32_t)wrap1(z0 - 1, P.nz) * plane + c].x;
+            V2<R> f = field[(uint32_t)z0 * plane + c];
+            uint32_t broken = 0;
 #pragma unroll 1
-        for (int z = z0; z < z1; ++z) {
-            const uint32_t pl = (uint32_t)z * plane;
-            const V2<R> f_p = field[(uint32_t)wrap1(z + 1, P.nz) * plane + c];
-            const V4<R> u = fluid[pl + c];
-            const R phi = f.x, pi = f.y;
-            R grad2 = R(0);
-            {
-                const R d = R(0.5) * (field[pl + cxp].x - field[pl + cxm].x) * P.inv_dx;
-                grad2 = grad2 + d * d;
+            for (int z = z0; z < z1; ++z) {
+                const uint32_t pl = (uint32_t)z * plane;
+                const V2<R> f_p = field[(uint32_t)wrap1(z + 1, P.nz) * plane + c];
+                const V4<R> u = fluid[pl + c];
+                const R phi = f.x, pi = f.y;
+                R grad2 = R(0);
+                {
+                    const R d = R(0.5) * (field[pl + cxp].x - field[pl + cxm].x) * P.inv_dx;
+                    grad2 = grad2 + d * d;
+                }
+                {
+                    const R d = R(0.5) * (field[pl + cyp].x - field[pl + cym].x) * P.inv_dx;
+                    grad2 = grad2 + d * d;
+                }
+                {
+                    const R d = R(0.5) * (f_p.x - phi_m) * P.inv_dx;
+                    grad2 = grad2 + d * d;
+                }
+                // In the perturbation form e_lab is max(E, e_floor) - e_bg: the sums of
+                // e_total and e_lab then miss N e_bg, which the host adds in FP64.
+                const R e_lab = vmax(u.x, P.e_floor);
+                const V4<R> q = diag_recover<R, MIXED>(u, P, phi);
+                const R v2 = q.x * q.x + q.y * q.y + q.z * q.z;
+                // the thermal form's field holds V(phi, 0); the rest of V(phi, T) is in E
+                R pot;
+                if constexpr (MIXED == kThermal) pot = thermal_potential0(phi, P);
+                else pot = diag_potential(phi, P);
+                const R e_total = R(0.5) * pi * pi + R(0.5) * grad2 + pot + e_lab;
+                R kinetic;
+                if constexpr (MIXED == kPert) kinetic = ((e_lab + q.w) + (P.e_bg + P.p_bg)) * v2;
+                else kinetic = (e_lab + q.w) * v2;
+                if constexpr (!WIDE) {
+                    s_total.add(e_total);
+                    s_kinetic.add(kinetic);
+                    s_e.add(e_lab);
+                } else {
+                    acc[0] += (double)e_total;
+                    acc[2] += (double)kinetic;
+                    acc[3] += (double)e_lab;
+                }
+                broken += phi > R(0.5) * P.phi_b ? 1u : 0u;
+                v2max = vmax(v2max, v2);
+                // max(E, e_floor) hides a NaN in E, so the raw state is checked too.
+                if (!isfinite(e_total) || !isfinite(v2) || !isfinite(f.x + f.y + u.x + u.y + u.z + u.w)) bad = 1;
+                phi_m = phi;
+                f = f_p;
             }
-            {
-                const R d = R(0.5) * (field[pl + cyp].x - field[pl + cym].x) * P.inv_dx;
-                grad2 = grad2 + d * d;
-            }
-            {
-                const R d = R(0.5) * (f_p.x - phi_m) * P.inv_dx;
-                grad2 = grad2 + d * d;
-            }
-            // In the perturbation form e_lab is max(E, e_floor) - e_bg: the sums of
-            // e_total and e_lab then miss N e_bg, which the host adds in FP64.
-            const R e_lab = vmax(u.x, P.e_floor);
-            const V4<R> q = diag_recover<R, MIXED>(u, P, phi);
-            const R v2 = q.x * q.x + q.y * q.y + q.z * q.z;
-            // the thermal form's field holds V(phi, 0); the rest of V(phi, T) is in E
-            R pot;
-            if constexpr (MIXED == kThermal) pot = thermal_potential0(phi, P);
-            else pot = diag_potential(phi, P);
-            const R e_total = R(0.5) * pi * pi + R(0.5) * grad2 + pot + e_lab;
-            R kinetic;
-            if constexpr (MIXED == kPert) kinetic = ((e_lab + q.w) + (P.e_bg + P.p_bg)) * v2;
-            else kinetic = (e_lab + q.w) * v2;
-            s_total.add(e_total);
-            s_kinetic.add(kinetic);
-            s_e.add(e_lab);
-            broken += phi > R(0.5) * P.phi_b ? 1u : 0u;
-            v2max = vmax(v2max, v2);
-            // max(E, e_floor) hides a NaN in E, so the raw state is checked too.
-            if (!isfinite(e_total) || !isfinite(v2) || !isfinite(f.x + f.y + u.x + u.y + u.z + u.w)) bad = 1;
-            phi_m = phi;
-            f = f_p;
+            return broken;
+        };
+        acc[1] += (double)march(std::false_type{});
+        if (sizeof(R) == 4 && !isfinite(s_total.hi + s_kinetic.hi + s_e.hi)) {
+            march(std::true_type{});
+        } else {
+            acc[0] += (double)s_total.hi + (double)s_total.lo;
+            acc[2] += (double)s_kinetic.hi + (double)s_kinetic.lo;
+            acc[3] += (double)s_e.hi + (double)s_e.lo;
         }
-        acc[0] += s_total.take();
-        acc[1] += (double)broken;
-        acc[2] += s_kinetic.take();
-        acc[3] += s_e.take();
     }
     float vmaxv = (float)sqrt(v2max);
     if (!isfinite(vmaxv)) bad = 1;
