@@ -186,12 +186,19 @@ template <typename R>
 struct PrimParts {
     R zx, zy, zz, p, s;
 };
+// z2 < c for z2 >= 0 (or NaN) and c >= 0
+template <typename R>
+BUBBLE_DEV bool below(R z2, R c) {
+    if constexpr (sizeof(R) == 8) return __double_as_longlong(z2) < __double_as_longlong(c);
+    else return z2 < c;
+}
 // |Z|^2 capped at zcap^2, Z scaled with it.  A |Z|^2 a hundredth below the cap's
-// square decides the comparison without the root.
+// square decides the comparison without the root (where both squares overflow
+// it is not below, and the roots are compared).
 template <typename R>
 BUBBLE_DEV R capped_z2(R &zx, R &zy, R &zz, R zcap) {
     R z2 = zx * zx + zy * zy + zz * zz;
-    if (above(z2, R(0.99) * (zcap * zcap))) {
+    if (!below(z2, R(0.99) * (zcap * zcap))) {
         const R zlen = sqrt(z2);
         if (above(zlen, zcap)) {
             const R s = zcap / vmax(zlen, R(1e-30));

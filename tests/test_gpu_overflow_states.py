@@ -1,0 +1,48 @@
+"""States whose squares overflow or that hold NaN, against the oracle.
+
+The strict and FP64 forms restate the oracle's arithmetic operation for
+operation, so they give its values also where E^2 and Z^2 are infinite and
+where a cell is NaN: equal finite values, and infinities and NaN in the same
+places.
+"""
+from __future__ import annotations
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+GRID = (24, 20, 18)
+
+
+def _step_both(bubble, oracle_mod, precision, f0, u0):
+    o = oracle_mod.OracleSim(GRID, precision={"single": "f32", "double": "f64", "perturbation": "pert"}[precision])
+    o.set_state(f0, u0)
+    o.advance(1)
+    spec = bubble.SimulationSpec(grid=GRID, bubbles=0, nucleation="centre", precision=precision, math="strict")
+    with bubble.Simulation(spec) as sim:
+        sim.load_state(f0, u0)
+        sim.advance(1)
+        got = sim.copy_state()
+    for a, s in zip(got, o.state()):
+        assert np.array_equal(a, s, equal_nan=True), np.argwhere((a != s) & ~(np.isnan(a) & np.isnan(s)))[:5]
+
+
+def _state(scale, dtype):
+    nx, ny, nz = GRID
+    n = nx * ny * nz
+    rng = np.random.default_rng(6)
+    d = rng.normal(size=(n, 3))
+    d /= np.linalg.norm(d, axis=1)[:, None]
+    e = scale * rng.uniform(0.9, 1.1, n)
+    z = d * (e * rng.choice([0.0, 0.3, 0.9999, 1.2, 3.0], size=n))[:, None]
+    field = np.zeros((n, 2))
+    fluid = np.concatenate([e[:, None], z], 1)
+    return field.astype(dtype), fluid.astype(dtype)
+
+
+@pytest.mark.parametrize("precision,scale", [("single", 3e18), ("single", 1e19), ("single", 3e19), ("perturbation", 1e19),
+                                             ("perturbation", 3e19), ("double", 1e154)])
+def test_energies_whose_squares_overflow(bubble, oracle_mod, gpu, precision, scale):
+    f0, u0 = _state(scale, np.float64 if precision == "double" else np.float32)
+    _step_both(bubble, oracle_mod, precision, f0, u0)
