@@ -100,8 +100,8 @@ BUBBLE_DEV double d_max_zero(double a) {                                        
     const long long x = __double_as_longlong(a);
     return x > 0 && x <= kInfBits ? a : 0.0;
 }
-BUBBLE_DEV double d_min_pos(double a, double c) {  // fmin(a, c) for a >= 0 (or NaN), c > 0
-    return __double_as_longlong(a) < __double_as_longlong(c) ? a : c;
+BUBBLE_DEV double d_min_pos(double a, double c) {  // fmin(a, c) for a >= +0 (or NaN of either sign), c > 0
+    return (unsigned long long)__double_as_longlong(a) < (unsigned long long)__double_as_longlong(c) ? a : c;
 }
 template <typename R>
 BUBBLE_DEV R max_pos(R a, R c) {  // max(a, c) for c > 0

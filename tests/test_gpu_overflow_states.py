@@ -46,3 +46,20 @@ def _state(scale, dtype):
 def test_energies_whose_squares_overflow(bubble, oracle_mod, gpu, precision, scale):
     f0, u0 = _state(scale, np.float64 if precision == "double" else np.float32)
     _step_both(bubble, oracle_mod, precision, f0, u0)
+
+
+@pytest.mark.parametrize("precision", ["single", "double"])
+@pytest.mark.parametrize("component", range(6))
+def test_cells_that_are_not_finite(bubble, oracle_mod, gpu, precision, component):
+    """NaN of either sign and infinities in one component of far-apart cells (an
+    infinite E is left out: there the strict kernels and the oracle differ
+    three cells away)."""
+    dtype = np.float64 if precision == "double" else np.float32
+    f0, u0 = _state(0.125, dtype)
+    u0[:, 1:] *= 0.3
+    nx, ny, _ = GRID
+    values = [np.nan, np.copysign(np.nan, -1.0)] + ([np.inf, -np.inf] if component != 2 else [])
+    for k, v in enumerate(values):
+        cell = ((4 * k + 3) * ny + 4 * k + 2) * nx + 5 * k + 1
+        (f0 if component < 2 else u0)[cell, component % 4 if component < 2 else component - 2] = v
+    _step_both(bubble, oracle_mod, precision, f0, u0)
