@@ -78,9 +78,11 @@ struct BubbleBatch {
 // brick's centre minus its half extent -- the periodic distance is
 // 1-Lipschitz) whose tanh argument exceeds the cut-off by a margin rules a
 // bubble out, its profile being exactly 0 in the whole brick.  The bound is
-// evaluated in FP32 and shortened by 4e-3 cells, more than its rounding on
-// axes of 2048 cells (in FP64, at two operations per clock and SM, the bounds
-// alone took half of a launch of 128 bubbles).  Every cell then takes max(phi,
+// evaluated in FP32 and shortened by more than its rounding: 4e-3 cells for
+// axes of 2048 cells and 2e-6 of the centre's coordinates and the radius, which
+// are the caller's and may lie far outside (in FP64, at two operations per clock
+// and SM, the bounds alone took half of a launch of 128 bubbles).  A bound whose
+// square leaves the FP32 range rules nothing out.  Every cell then takes max(phi,
 // 0), the far field of all the batch's bubbles, and the maximum over the kept
 // bubbles alone, in any order: the result equals the reference's loop over the
 // whole batch bit for bit.  A thread's eight cells are loaded together, and a
@@ -114,8 +116,9 @@ __global__ void __launch_bounds__(256) nucleate_kernel(V2<R> *__restrict__ field
             const float g = fmaxf(fabsf(d) - half, 0.0f);
             lb2 += g * g;
         }
-        const float arg_lb = ((sqrtf(lb2) - 4e-3f) * (float)P.dx - bub.w * (float)P.dx) / (float)P.wall_width;
-        if (!(arg_lb > (float)cut + 0.25f)) kept[atomicAdd(&n_kept, 1)] = b;
+        const float slack = 4e-3f + 2e-6f * (fabsf(c[0]) + fabsf(c[1]) + fabsf(c[2]) + fabsf(bub.w));
+        const float arg_lb = (sqrtf(lb2) - bub.w - slack) * (float)P.dx / (float)P.wall_width;
+        if (!(arg_lb > (float)cut + 0.25f && lb2 < 1e38f)) kept[atomicAdd(&n_kept, 1)] = b;
     }
     __syncthreads();
     const int nk = n_kept;
