@@ -34,25 +34,34 @@ BUBBLE_DEV float2 sqrt2(float2 a) { return make_float2(sqrt_approx(a.x), sqrt_ap
 BUBBLE_DEV float2 max2(float2 a, float s) { return make_float2(fmaxf(a.x, s), fmaxf(a.y, s)); }
 BUBBLE_DEV float2 dot3_2(float2 x, float2 y, float2 z) { return p_fma(z, z, p_fma(y, y, p_mul(x, x))); }
 
-// min(|a|, |b|) with the product of the signs
+// min(|a|, |b|) with the product of the signs; the other operand, or (KEEP_NAN) NaN,
+// where one is NaN
+template <bool KEEP_NAN = false>
 BUBBLE_DEV float min_xorsign(float a, float b) {
     float r;
-    asm("min.xorsign.abs.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
+    if constexpr (KEEP_NAN) asm("min.NaN.xorsign.abs.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
+    else asm("min.xorsign.abs.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
     return r;
 }
-// the smaller of both, NaN if either is
+// the smaller, the larger of both, NaN if either is
 BUBBLE_DEV float min_nan(float a, float b) {
     float r;
     asm("min.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
+    return r;
+}
+BUBBLE_DEV float max_nan(float a, float b) {
+    float r;
+    asm("max.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
     return r;
 }
 
 // Half of the MC-limited slope (limit_slope): 0 unless dm and dp have one
 // sign, else min(|dm + dp| / 4, |dm|, |dp|) with it.  The signed minimum
 // min(|dm|, |dp|) sign(dm dp), floored at 0, is 0 exactly when the signs
-// differ, so no comparison is needed: three instructions per value.
+// differ, so no comparison is needed: three instructions per value.  0 also
+// beside a cell that is NaN, so NaN spreads no further than the stencil.
 BUBBLE_DEV float half_slope(float dm, float dp, float quarter_sum) {
-    return min_xorsign(quarter_sum, fmaxf(min_xorsign(dm, dp), 0.0f));
+    return min_xorsign(quarter_sum, fmaxf(min_xorsign<true>(dm, dp), 0.0f));
 }
 BUBBLE_DEV float2 half_slope2(float2 qm, float2 q, float2 qp) {
     const float2 dm = p_sub(q, qm), dp = p_sub(qp, q);
@@ -183,7 +192,7 @@ static __device__ __noinline__ V4<float> recover_slow_thermal(V4<float> u, float
 // scheduled between them: recover_pair evaluates both cells by the formulas
 // that hold below gamma = 3 and above the pressure floor, which it does not
 // apply; recover_fix sends a cell whose |v|^2 came out above 8/9 (gamma > 3)
-// or whose p is below the floor or NaN through the scalar recovery.  Together
+// or NaN, or whose p is below the floor or NaN, through the scalar recovery.  Together
 // they cover every cell whose |Z| exceeds z_max E: the uncapped p of the bag
 // forms and the gamma law is then below the floor, NaN, or so small that |v|^2
 // is above 8/9 (where the floor is comparable to E, |v| alone can stay below);
@@ -265,7 +274,7 @@ BUBBLE_DEV void recover_fix(P4 &q, const V4<float> *ua, const V4<float> *ub, flo
     const float2 v2 = dot3_2(q.x, q.y, q.z);
     constexpr float kFast = 8.0f / 9.0f;
     // (the thermal form floors p and marks the cells itself)
-    if (fmaxf(v2.x, v2.y) > kFast || (FORM != kThermal && !(min_nan(q.w.x, q.w.y) >= P.p_floor))) {
+    if (!(max_nan(v2.x, v2.y) <= kFast) || (FORM != kThermal && !(min_nan(q.w.x, q.w.y) >= P.p_floor))) {
         auto slow = [&](const V4<float> *u, float f) {
             if constexpr (FORM == kThermal)
                 return recover_slow_thermal(*u, f, P.e_floor, P.z_max, P.p_floor, P.th_k, P.th_g, P.th_h, P.th_i2a,
@@ -274,14 +283,14 @@ BUBBLE_DEV void recover_fix(P4 &q, const V4<float> *ua, const V4<float> *ub, flo
                 return recover_slow<FORM>(*u, P.e_floor, P.z_max, P.p_floor, FORM == kGamma ? P.eos_c2 : P.e_bg,
                                           FORM == kGamma ? P.eos_e0 : P.p_bg);
         };
-        if (v2.x > kFast || !(q.w.x >= P.p_floor)) {
+        if (!(v2.x <= kFast) || !(q.w.x >= P.p_floor)) {
             const V4<float> r = slow(ua, phi.x);
             q.x.x = r.x;
             q.y.x = r.y;
             q.z.x = r.z;
             q.w.x = r.w;
         }
-        if (v2.y > kFast || !(q.w.y >= P.p_floor)) {
+        if (!(v2.y <= kFast) || !(q.w.y >= P.p_floor)) {
             const V4<float> r = slow(ub, phi.y);
             q.x.y = r.x;
             q.y.y = r.y;
@@ -382,10 +391,12 @@ struct FacePair {
 BUBBLE_DEV FacePair face_pair(const P4 &l, const P4 &r, float2 fl, float2 fr, bool exchanged = false) {
     return FacePair{l, r, speed2(l, exchanged), speed2(r, exchanged), fl, fr};
 }
-BUBBLE_DEV float max_speed2(const FacePair &f) {
-    return fmaxf(fmaxf(f.vl.x, f.vl.y), fmaxf(f.vr.x, f.vr.y));
+// Whether a speed of a face pair is beyond the cap or NaN.
+BUBBLE_DEV bool needs_clamp(const FacePair &f, float zmax2) {
+    return !(max_nan(max_nan(f.vl.x, f.vl.y), max_nan(f.vr.x, f.vr.y)) <= zmax2);
 }
-// The velocity clamps of a face pair one of whose speeds is beyond the cap.
+// The velocity clamps of such a pair; |v|^2 of a NaN velocity is the cap's, so
+// the components that are not NaN keep finite fluxes.
 BUBBLE_DEV void clamp_face(FacePair &f, float zmax2, bool exchanged = false) {
     clamp_pair(f.l, f.vl, zmax2, exchanged);
     clamp_pair(f.r, f.vr, zmax2, exchanged);

@@ -339,7 +339,7 @@ BUBBLE_DEV bool pair_item(unsigned char *smem, const StageArgs<float> &A, const 
                 P4 lo, up;
                 face_states_pair(q0, q1, q2, P.p_floor, lo, up);
                 FacePair f = face_pair(hiz, lo, phi_at(z, 0), phi_at(z + 1, 0));
-                if (max_speed2(f) > zmax2) clamp_face(f, zmax2);
+                if (needs_clamp(f, zmax2)) clamp_face(f, zmax2);
                 fz_p = hll_pair<2, FORM>(f, P);
                 hiz = up;
             }
@@ -355,7 +355,7 @@ BUBBLE_DEV bool pair_item(unsigned char *smem, const StageArgs<float> &A, const 
             const uint32_t base = (uint32_t)z * plane;
             if constexpr (ACT) {
                 FacePair f = face_pair(get_pair<FX>(hx, ix), lox, phi_at(z, -1), phi_at(z, 0));
-                if (max_speed2(f) > zmax2) clamp_face(f, zmax2);
+                if (needs_clamp(f, zmax2)) clamp_face(f, zmax2);
                 put_pair<FX>(fx, ix, hll_pair<0, FORM>(f, P));
                 // cells beyond the edge load their wrapped images and are not stored
                 pf0 = A.field_in[base + g0];
@@ -369,7 +369,7 @@ BUBBLE_DEV bool pair_item(unsigned char *smem, const StageArgs<float> &A, const 
                     un1 = A.fluid_n[base + g1];
                 }
                 f = face_pair(get_pair<FY>(hy, iy), loy, phi_at(z, -PQ), phi_at(z, 0));
-                if (max_speed2(f) > zmax2) clamp_face(f, zmax2);
+                if (needs_clamp(f, zmax2)) clamp_face(f, zmax2);
                 yl = hll_pair<1, FORM>(f, P);
                 put_pair<FY>(fy, iy, yl);
                 if (cj == 0) put_half<FY, 1, 0>(fy, 8 * 16 + ci, yl);  // face 8 is also the first half of face pair 8
@@ -524,7 +524,7 @@ BUBBLE_DEV bool pair_item(unsigned char *smem, const StageArgs<float> &A, const 
                     }
                 }
                 FacePair f = face_pair(l, r, pl, pq, !xf);
-                if (max_speed2(f) > zmax2) clamp_face(f, zmax2, !xf);
+                if (needs_clamp(f, zmax2)) clamp_face(f, zmax2, !xf);
                 P4 fl = hll_pair<0, FORM>(f, P);
                 if (xf) {
                     put_pair<FX>(fx, h * FXW + 16, fl);

@@ -166,3 +166,31 @@ def test_thermal_temperature_off_the_branch(bubble, gpu, phi):
     strict, fast = _pi_after_a_step(bubble, states, (gamma, a), pi=0.0)
     err = np.max(np.abs(fast - strict), axis=1) / np.max(np.abs(strict), axis=1)
     assert np.all(err <= 1e-5), [(states[k], err[k]) for k in np.flatnonzero(err > 1e-5)]
+
+
+@pytest.mark.parametrize("precision,eos,eos_param", [("single", "bag", (1.0, 0.0)), ("mixed", "bag", (1.0, 0.0)),
+                                                     ("perturbation", "bag", (1.0, 0.0)),
+                                                     ("single", "gamma_law", (1.2, 0.05)),
+                                                     ("single", "thermal", (0.0125, 0.05))])
+@pytest.mark.parametrize("component", range(6))
+def test_nan_spreads_as_in_the_strict_form(bubble, gpu, component, precision, eos, eos_param):
+    """A NaN in one component of a cell reaches the same values after a step,
+    and the others are those of the strict form."""
+    nx, ny, nz = GRID
+    n = nx * ny * nz
+    rng = np.random.default_rng(7)
+    e = E_REF * rng.uniform(0.8, 1.2, n) - (E_REF if precision == "perturbation" else 0.0)
+    f0, u0 = _state(e, E_REF * rng.uniform(-0.1, 0.1, (n, 3)), rng.uniform(-0.1, 1.1, n), rng.normal(0, 0.02, n))
+    (f0 if component < 2 else u0)[(9 * ny + 10) * nx + 11, component % 4 if component < 2 else component - 2] = np.nan
+    got = {}
+    for math in ("strict", "fast"):
+        spec = bubble.SimulationSpec(grid=GRID, bubbles=0, nucleation="centre", precision=precision, math=math, eos=eos,
+                                     eos_param=eos_param)
+        with bubble.Simulation(spec) as sim:
+            sim.load_state(f0, u0)
+            sim.advance(1)
+            got[math] = np.concatenate(sim.copy_state(), axis=1).astype(np.float64)
+    s, a = got["strict"], got["fast"]
+    assert np.array_equal(np.isnan(a), np.isnan(s))
+    err = np.nanmax(np.abs(a - s), axis=0) / np.nanmax(np.abs(s), axis=0)
+    assert np.all(err <= 1e-5), err
