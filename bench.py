@@ -660,7 +660,7 @@ def main() -> int:
     # warm-up: nucleation at t = 0 plus W steps
     sim.advance(args.warmup)
     sim.synchronize()
-    ty, lz = sim.tile()
+    ty, lz = sim.tile()[0], sim.chunk()
 
     def barrier():
         if pg:

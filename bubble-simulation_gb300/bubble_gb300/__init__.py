@@ -227,6 +227,12 @@ class Simulation:
         check(self._L.bubble_ext_get_tile(self._h, ctypes.byref(ty), ctypes.byref(lz)))
         return ty.value, lz.value
 
+    def chunk(self) -> int:
+        """Planes marched per CTA by the fused kernel's launches."""
+        lz = ctypes.c_int32()
+        check(self._L.bubble_ext_get_chunk(self._h, ctypes.byref(lz)))
+        return lz.value
+
     # -- stepping -------------------------------------------------------------
     def record_steps(self, n: int = 1):
         check(self._L.bubble_record_steps(self._h, n))

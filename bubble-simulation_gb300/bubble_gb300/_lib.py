@@ -185,6 +185,7 @@ SIGNATURES = [
     ("bubble_ext_set_path", ctypes.c_int, [_P, ctypes.c_int32]),
     ("bubble_ext_set_tile", ctypes.c_int, [_P, ctypes.c_int32, ctypes.c_int32]),
     ("bubble_ext_get_tile", ctypes.c_int, [_P, _I32P, _I32P]),
+    ("bubble_ext_get_chunk", ctypes.c_int, [_P, _I32P]),
     ("bubble_ext_set_stage_form", ctypes.c_int, [_P, ctypes.c_int32]),
     ("bubble_ext_device_state", ctypes.c_int, [_P, ctypes.POINTER(_P), ctypes.POINTER(_P)]),
     ("bubble_ext_stream", _P, [_P]),

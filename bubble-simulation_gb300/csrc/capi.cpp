@@ -314,6 +314,11 @@ int bubble_ext_get_tile(const bubble_sim *sim, int32_t *ty, int32_t *lz) {
     if (lz) *lz = t.lz;
     return BUBBLE_OK;
 }
+int bubble_ext_get_chunk(const bubble_sim *sim, int32_t *lz) {
+    if (!sim || !sim->impl) return fail(BUBBLE_ERR_INVALID, "sim is NULL");
+    if (lz) *lz = sim->impl->chunk();
+    return BUBBLE_OK;
+}
 int bubble_ext_device_state(bubble_sim *sim, void **field, void **fluid) {
     if (!sim || !sim->impl) return fail(BUBBLE_ERR_INVALID, "sim is NULL");
     sim->impl->device_state(field, fluid);

@@ -432,9 +432,17 @@ int Simulation::set_tile(TileShape t, std::string &err) {
             tma_ok_ = tma_ok_ && encode_stage_maps(&maps_[k], field_[k], fluid_[k], (int)grid_[0], (int)grid_[1],
                                                    (int)grid_[2], t.tx, t.ty, is_f64() ? 8 : 4);
     }
+    // The chunk that get_tile reports by default stands for the arithmetic's own
+    // pick, so setting a reported tile changes nothing.
+    if (!is_f64() && t.ty == 16 && t.pair_lz == 0 && t.lz == default_chunk(grid_, 16, true)) t.pair_lz = pair_chunk(grid_);
     t.form = tile_.form;
     tile_ = t;
     return BUBBLE_OK;
+}
+
+int Simulation::chunk() const {
+    const bool pair = !is_f64() && spec_.math == BUBBLE_MATH_FAST && tile_.ty == 16;
+    return pair && tile_.pair_lz > 0 ? tile_.pair_lz : tile_.lz;
 }
 
 int Simulation::set_stage_form(int form, std::string &err) {

@@ -61,10 +61,13 @@ class Simulation {
         test_shift_ = shift;
     }
     KernelPath path() const { return path_; }
-    int set_tile(TileShape t, std::string &err);  // keeps the stage form
+    // Keeps the stage form; pair_lz 0: lz, or the pair form's own pick where lz
+    // is the default.
+    int set_tile(TileShape t, std::string &err);
     // BUBBLE_STAGE_FORM_* of FP32 16 x 16 launches
     int set_stage_form(int form, std::string &err);
     TileShape tile() const { return tile_; }
+    int chunk() const;  // planes per CTA of the fused stage launches
 
     float time() const { return time_; }
     uint64_t steps() const { return steps_; }

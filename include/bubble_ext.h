@@ -27,9 +27,12 @@ int bubble_ext_set_path(bubble_sim *sim, int32_t path);
  * and MIXED forms; 4 for 32 x 4 in those forms with the fast arithmetic;
  * FP64: 16 (default) or 4 for 32 x 4) and z chunk (planes marched per CTA).
  * Until it is set, the fast arithmetic picks a chunk of its own and the chunk
- * reported is the column kernel's. */
+ * reported is the column kernel's; setting that one keeps, or brings back, the
+ * own pick. */
 int bubble_ext_set_tile(bubble_sim *sim, int32_t ty, int32_t lz);
 int bubble_ext_get_tile(const bubble_sim *sim, int32_t *ty, int32_t *lz);
+/* Planes marched per CTA by the fused kernel's launches as they are now. */
+int bubble_ext_get_chunk(const bubble_sim *sim, int32_t *lz);
 
 /* Form of the fused column kernel for FP32 16 x 16 tiles; both forms give
  * identical bits.  The fast arithmetic has one form of its own, two cells per
