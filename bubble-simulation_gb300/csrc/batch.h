@@ -143,8 +143,9 @@ class Batch {
     bool dirty_ = true;  // membership changed since the last plan_items()
 };
 
-// Fastest z chunk of the fused stage kernel for one lattice size, measured
-// on the device (cached per size, tile height and arithmetic mode).
-int autotune_chunk(const uint32_t grid[3], int ty, bool fast, std::string &err);
+// Fastest z chunk, of those of `shortest` planes and more, of the fused stage
+// kernel for one lattice size, measured on the device (cached per size, tile
+// height and arithmetic mode).
+int autotune_chunk(const uint32_t grid[3], int ty, bool fast, int shortest, std::string &err);
 
 }  // namespace bubble

@@ -82,7 +82,7 @@ int bubble_ext_test_expire_batch_barrier(bubble_batch *batch, int32_t wait_shift
 int bubble_autotune_chunk(const uint32_t grid[3], int32_t tile_y, int32_t math, int32_t *lz_out) {
     if (!grid || !lz_out) return fail(BUBBLE_ERR_INVALID, "grid and lz_out must be non-NULL");
     std::string err;
-    const int lz = bubble::autotune_chunk(grid, tile_y, math == BUBBLE_MATH_FAST, err);
+    const int lz = bubble::autotune_chunk(grid, tile_y, math == BUBBLE_MATH_FAST, 1, err);
     if (lz <= 0) return fail(BUBBLE_ERR_CUDA, err.empty() ? "autotune failed" : err);
     *lz_out = lz;
     return BUBBLE_OK;
