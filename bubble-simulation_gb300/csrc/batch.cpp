@@ -6,12 +6,12 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
-#include <functional>
 #include <mutex>
 #include <numeric>
 #include <utility>
 #include <vector>
 
+#include "chunk_plan.h"
 #include "launch.h"
 #include "simulation.h"
 
@@ -349,88 +349,6 @@ int Batch::remove(uint32_t k, std::string &err) {
     return BUBBLE_OK;
 }
 
-// Chunks of the shared lattices for the shortest round.  Equal chunks per
-// lattice, no longer than one cap for the first (largest) lattices and a
-// smaller one for the rest, whose short items fill the round's end; among
-// such plans with caps up to cap_max, the one whose round ends first when its
-// items, each its planes and its warm-up's, are handed out in order to the
-// persistent CTAs as they come free.  Any chunking gives the same bits.  The
-// estimate before, the work spread evenly plus the longest item, counted every
-// round's end as a whole item, so it cut too finely, and knew one cap: 16 short
-// solves of 48^3 .. 128^3 were served in 60.8 ms then, in 57.5 ms now, a light
-// stream of 24 at 9.35 solves/s then, at 10.08 now.
-std::vector<int> Batch::balanced_chunks(int cap_max) const {
-    const bool pair = fast_ && ty_ == 16;
-    const double warm_up = pair ? 1.6 : 2.0;  // planes, as in the launch cost models (params.h)
-    const int tx = tile_x_for(ty_);
-    const size_t n = item_order_.size();
-    auto lz_of = [](const Lat &L, int cap) {
-        const int nz = (int)L.grid[2];
-        const int pieces = (nz + cap - 1) / cap;
-        return (nz + pieces - 1) / pieces;
-    };
-    std::vector<std::pair<double, int>> busy;  // (time, CTAs that come free then), a heap
-    auto round_time = [&](int cap_a, int cap_b, size_t split) {
-        const auto later = std::greater<std::pair<double, int>>();
-        busy.assign(1, {0.0, std::max(1, max_grid_)});
-        double end = 0.0;
-        long total = 0;
-        for (size_t q = 0; q < n;) {
-            const Lat &L = lats_[item_order_[q]];
-            const int lz = lz_of(L, q < split ? cap_a : cap_b);
-            const long tiles = (long)((L.grid[0] + tx - 1) / tx) * (long)((L.grid[1] + ty_ - 1) / ty_);
-            long items = 0;  // of this lattice and of those like it behind it
-            for (; q < n; ++q) {
-                const Lat &M = lats_[item_order_[q]];
-                if (std::memcmp(M.grid, L.grid, sizeof(L.grid)) != 0 || lz_of(M, q < split ? cap_a : cap_b) != lz)
-                    break;
-                items += tiles * (((long)L.grid[2] + lz - 1) / lz);
-            }
-            total += items;
-            while (items > 0) {
-                std::pop_heap(busy.begin(), busy.end(), later);
-                const auto [t, ctas] = busy.back();
-                busy.pop_back();
-                const int take = (int)std::min<long>(items, ctas);
-                items -= take;
-                end = std::max(end, t + lz + warm_up);
-                busy.emplace_back(t + lz + warm_up, take);
-                std::push_heap(busy.begin(), busy.end(), later);
-                if (take < ctas) {
-                    busy.emplace_back(t, ctas - take);
-                    std::push_heap(busy.begin(), busy.end(), later);
-                }
-            }
-        }
-        // CTAs with an SM to themselves, or shared by two, are faster
-        if (pair && 3 * total <= max_grid_) return 0.57 * end;
-        if (pair && 3 * total <= 2 * (long)max_grid_) return 0.77 * end;
-        return end;
-    };
-    double best = 1e300;
-    int best_a = cap_max, best_b = cap_max;
-    size_t best_split = n;
-    auto consider = [&](int cap_a, int cap_b, size_t split) {
-        const double cost = round_time(cap_a, cap_b, split);
-        if (cost < best * (1.0 - 1e-9)) {
-            best = cost;
-            best_a = cap_a;
-            best_b = cap_b;
-            best_split = split;
-        }
-    };
-    for (int cap : {cap_max, 48, 32, 24, 16, 12, 8, 6, 4}) {
-        if (cap > cap_max) continue;
-        consider(cap, cap, n);
-        for (int rest : {16, 8, 4})
-            for (size_t split : {n / 4, n / 2, 3 * n / 4})
-                if (rest < cap && split > 0) consider(cap, rest, split);
-    }
-    std::vector<int> lz(n);
-    for (size_t q = 0; q < n; ++q) lz[q] = lz_of(lats_[item_order_[q]], q < best_split ? best_a : best_b);
-    return lz;
-}
-
 // Items of a stage for the active lattices (largest first) and the grid.
 void Batch::plan_items() {
     item_order_.clear();
@@ -449,7 +367,9 @@ void Batch::plan_items() {
         return n;
     };
     if (fill_) {
-        const std::vector<int> lz = balanced_chunks(lz_cap_);
+        std::vector<ChunkPlanGrid> grids;
+        for (uint32_t k : item_order_) grids.push_back({lats_[k].grid[0], lats_[k].grid[1], lats_[k].grid[2]});
+        const std::vector<int> lz = balanced_chunks(grids, tx, ty_, fast_ && ty_ == 16, max_grid_, lz_cap_);
         for (size_t q = 0; q < lz.size(); ++q) lats_[item_order_[q]].lz = lz[q];
     }
     n_items_ = count_items();

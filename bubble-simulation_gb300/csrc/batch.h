@@ -91,7 +91,6 @@ class Batch {
     int launch_solo(Lat &L, uint64_t k, std::string &err);
     int autotune(std::string &err);
     void plan_items();
-    std::vector<int> balanced_chunks(int cap_max) const;
     int ensure_capacity(size_t n, std::string &err);
     int check_status(std::string &err);
 
