@@ -53,7 +53,7 @@ std::mutex g_tune_mu;
 std::map<std::tuple<uint32_t, uint32_t, uint32_t, int, bool>, std::vector<std::pair<int, float>>> g_tune_cache;
 
 constexpr size_t kOffStatus = 64;     // counters at 0 (16 B), status at 64
-constexpr size_t kOffDiag = 256;      // diag partials | ticket | result
+constexpr size_t kOffDiag = 256;      // diag partials | ticket
 
 std::string check_spec(const bubble_spec &s, int math) {
     const std::string msg = validate_model(s.model);
@@ -180,7 +180,7 @@ int Batch::setup(int math, const bubble_batch_options *opt, std::string &err) {
     }
     BATCH_CUDA(cudaStreamCreateWithFlags(&stream_, cudaStreamNonBlocking), "cudaStreamCreate");
     const size_t pb = (launch::diag_partials_bytes() + 255) & ~(size_t)255;
-    const size_t scratch = kOffDiag + pb + 256 + 256;
+    const size_t scratch = kOffDiag + pb + 256;
     BATCH_CUDA(cudaMalloc(&d_scratch_, scratch), "cudaMalloc");
     BATCH_CUDA(cudaMemsetAsync(d_scratch_, 0, scratch, stream_), "cudaMemset");
     d_counters_ = static_cast<unsigned int *>(d_scratch_);

@@ -133,7 +133,7 @@ class Batch {
     BatchLattice *h_lat_ = nullptr;  // pinned
     unsigned int *d_counters_ = nullptr;
     int *d_status_ = nullptr;
-    void *d_scratch_ = nullptr;  // counters | status | diag partials | ticket | result
+    void *d_scratch_ = nullptr;  // counters | status | diag partials | ticket
     HostReport *h_report_ = nullptr;  // pinned
     cudaStream_t stream_ = nullptr;
     uint64_t launches_ = 0;

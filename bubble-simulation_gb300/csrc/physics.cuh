@@ -129,7 +129,9 @@ BUBBLE_DEV double d_max(double a, double b) { return d_nan(a) ? b : (d_nan(b) ||
 
 // Half of the MC-limited slope of limit_slope<double, false>: the minimum of
 // |dm + dp| / 4, |dm| and |dp| with their sign, 0 unless dm and dp have one.
-// Scaling by powers of two is exact, so q +- this is half_step's q +- s / 2.
+// Scaling by powers of two is exact, so q +- this is half_step's q +- s / 2 (the
+// quarter of a subnormal sum, rounded once instead of twice, can differ by its
+// last place, 5e-324).
 BUBBLE_DEV double d_half_slope(double dm, double dp) {
     const unsigned long long sign = 0x8000000000000000ull;
     const unsigned long long a = (unsigned long long)__double_as_longlong(dm), b = (unsigned long long)__double_as_longlong(dp);
@@ -254,8 +256,8 @@ BUBBLE_DEV V4<R> prim_from_cons(const V4<R> &u, const LatticeParams<R> &P) {
 // the FP32 state and constants by value, so it can also be compiled out of
 // line (BUBBLE_F64_RECOVERY_LINKAGE): one copy per kernel was 1.6 % faster
 // for the register-form stage kernel at 512^3 (fewer instruction-fetch
-// stalls), inlined is 0.6 % faster for the shared form, which now runs every
-// large lattice.
+// stalls), inlined is 0.6 % faster for the shared form, which runs the large
+// lattices of the strict arithmetic.
 #define BUBBLE_F64_RECOVERY_LINKAGE __device__ __forceinline__
 template <bool FAST = false>
 BUBBLE_F64_RECOVERY_LINKAGE V4<float> prim_from_cons_f64_x(V4<float> u, float e_floor, float z_max, float p_floor);

@@ -137,7 +137,7 @@ class Simulation {
     void *field_[3] = {nullptr, nullptr, nullptr};
     void *fluid_[3] = {nullptr, nullptr, nullptr};
     void *prim_ = nullptr;      // reference path only
-    void *scratch_ = nullptr;   // diag partials | ticket | result | status
+    void *scratch_ = nullptr;   // diag partials | ticket | status
     void *partials_ = nullptr;
     unsigned int *ticket_ = nullptr;
     int *d_status_ = nullptr;   // bit 0: a bounded wait in a stage kernel expired
@@ -170,8 +170,8 @@ int arith_mode(const bubble_spec &spec);
 
 // Default z chunk of the fused kernel for a lattice.  FP32 16 x 16 tiles:
 // the chunk whose cheaper form is cheapest under column_stage_cost (params.h);
-// FP64: the cheapest under fp64_stage_cost; otherwise enough CTAs to fill the GPU while keeping each chunk's warm-up a
-// small fraction of its work.
+// FP64: the cheapest under fp64_stage_cost; otherwise enough CTAs to fill the
+// GPU while keeping each chunk's warm-up a small fraction of its work.
 int default_chunk(const uint32_t grid[3], int ty, bool fp32);
 // z chunk of the pair form (stage_pair.cuh) where the caller set none: the
 // cheapest under pair_stage_cost (params.h).

@@ -135,7 +135,7 @@ BUBBLE_DEV void combine_cell(const StageArgs<R> &A, const LatticeParams<R> &P, u
     // plasma part, exchanged like the friction
     R dpot, src = drag;
     if constexpr (FORM == kThermal) {
-        const R T0 = thermal_temperature<R, FAST>(q0.w, phi0, P);
+        const R T0 = thermal_temperature<R, false>(q0.w, phi0, P);
         dpot = thermal_dpotential(phi0, T0, P);
         src = drag + thermal_exchange(phi0, T0, P);
     } else {
@@ -188,6 +188,8 @@ BUBBLE_DEV void combine_cell(const StageArgs<R> &A, const LatticeParams<R> &P, u
 template <typename R, bool FAST, int FORM, int TY, bool LEAN = false>
 BUBBLE_DEV bool column_item(unsigned char *smem, const StageArgs<R> &A, const LatticeParams<R> &P, int lz,
                         const StageMaps *maps, int tma_ok, int *status, int tile_xy, int chunk) {
+    static_assert(!FAST || (!LEAN && TY != 16 && (FORM == kPlain || FORM == kMixed)),
+                  "the fast arithmetic runs here on 32-wide tiles only");
     using L = ColumnLayout<R, TY, LEAN>;
     constexpr int TX = L::TX, NC = L::NC, NH = L::NH, PW = L::PW, PC = L::PC;
     __syncthreads();  // a previous item on this CTA is done with shared memory
