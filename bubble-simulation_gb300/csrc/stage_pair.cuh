@@ -17,7 +17,7 @@
 //
 // What bounds it.  The scalar column form issued 26.6 warp instructions per
 // cell and stage (256^3, MIXED) and was bound by that; the pair form issues
-// 16.2 (15.5 in the first stage).  Packed FP32 takes the FMA pipe as long as two scalar instructions
+// 16.4 (15.6 in the first stage).  Packed FP32 takes the FMA pipe as long as two scalar instructions
 // (0.36 fma.f32x2 and 0.49 add.f32x2 or mul.f32x2 per clock and scheduler,
 // measured, against 0.61 fma and 0.93 add), so it saves issue slots, not
 // arithmetic time: FMA pipe 50 %, shared-memory data path 63 %, issue 59 % at
@@ -30,7 +30,7 @@
 // mbarrier arrivals and waits around independent work (1 to 4 % slower), the
 // first stage in its own instantiation (1 % faster from 128^3, 1 % slower at
 // 64^3 and below, where two kernels alternate).  Step time, column form to
-// pair form (GB300): 512^3 MIXED 10.85 -> 8.25 ms, 256^3 perturbation 1.54 ->
+// pair form (GB300): 512^3 MIXED 10.85 -> 8.26 ms, 256^3 perturbation 1.54 ->
 // 1.16 ms, 128^3 0.212 -> 0.170 ms, 64^3 49.3 -> 43.1 us (0.160 ms and 36.5 us
 // with dependent launches and the form's own z chunk); the gamma law at 128^3,
 // with its recovery in closed form, 0.33 -> 0.18 ms, the thermal potential at
