@@ -326,7 +326,8 @@ BUBBLE_DEV bool column_item(unsigned char *smem, const StageArgs<R> &A, const La
     // Wait for raw plane p (`newer`: plane p+1 was issued after it); false
     // when the bounded wait expired.
     auto wait_raw = [&](int p, bool newer) -> bool {
-        if (tma) return mbar_wait_bounded(&bar[raw_slot(p)], ((p - z0) >> 1) & 1, A.wait_shift);
+        constexpr bool try_first = sizeof(R) == 8 || FAST;
+        if (tma) return mbar_wait_bounded<try_first>(&bar[raw_slot(p)], ((p - z0) >> 1) & 1, A.wait_shift);
         if (newer) cp_async_wait_but_one();
         else cp_async_wait_all();
         return true;

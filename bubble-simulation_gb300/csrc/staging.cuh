@@ -49,9 +49,13 @@ BUBBLE_DEV bool mbar_try_wait(uint64_t *bar, uint32_t parity) {
     return ok != 0;
 }
 // Bounded wait: gives up after 2^shift SM cycles (2^31 by default, about a
-// second at GB300 clocks).
+// second at GB300 clocks).  TRY_FIRST: a try before the clock is read, which the
+// pair, FP64 and 32-wide kernels run faster with (512^3 mixed 8.25 and 8.30 ms a
+// step) and the strict FP32 kernels slower (256^3 mixed 4.56 ms with, 4.47
+// without, perturbation 5.09 and 4.94, 64^3 71.7 and 69.0 us).
+template <bool TRY_FIRST = true>
 BUBBLE_DEV bool mbar_wait_bounded(uint64_t *bar, uint32_t parity, int shift) {
-    if (mbar_try_wait(bar, parity)) return true;
+    if (TRY_FIRST && mbar_try_wait(bar, parity)) return true;
     const long long start = clock64();
     const long long limit = 1ll << shift;
     while (!mbar_try_wait(bar, parity)) {
