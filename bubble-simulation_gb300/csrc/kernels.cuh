@@ -298,12 +298,23 @@ BUBBLE_DEV double warp_sum(double v) {
 
 constexpr int kDiagBlocksPerSm = 4;  // at 512^3: 2.07 ms with 3, 1.29 with 4, 1.40 with 5, 1.66 with 8
 
-// Planes of a chunk: about two items per SM on small lattices (one round of
-// blocks: 64^3 58 us a report at one plane, 39 at four), at most 32 planes.
-BUBBLE_HD int diag_planes(uint64_t nx, uint64_t ny, uint64_t nz) {
-    const uint64_t groups = (nx * ny + kDiagThreads - 1) / kDiagThreads;
-    const uint64_t lz = (groups * nz + 299) / 300;
-    return lz > 32 ? 32 : (int)lz;
+// Planes of a chunk.  Bag forms in FP32: about two items per SM on small lattices
+// (one round of blocks: 64^3 58 us a report at one plane, 39 at four), at most
+// 32 planes.  The Newton steps of the gamma law and the thermal potential and
+// the FP64 pipe make a plane several times as long, so there the even share of
+// the SMs decides and long items end unevenly (us a report, the bag forms' rule
+// and this one: gamma law 112^3 188 and 88, 128^3 306 and 163, 160^3 517 and 345,
+// 256^3 1271 and 1157; thermal potential 128^3 354 and 193; FP64 128^3 628 and
+// 517).  One plane up to 12288 plane groups: two planes take 284 us at 144^3
+// where one takes 244, and 345 at 160^3 where one takes 339 (on a lattice full
+// of walls 143 and 164).
+template <typename R, int MIXED>
+inline int diag_planes(uint64_t nx, uint64_t ny, uint64_t nz) {
+    const uint64_t groups = (nx * ny + kDiagThreads - 1) / kDiagThreads * nz;  // 256 cells of a plane each
+    const int lz = groups > 32 * 300 ? 32 : (int)((groups + 299) / 300);
+    if (sizeof(R) == 8) return groups > 1200 ? 3 : lz;
+    if (MIXED == kGamma || MIXED == kThermal) return groups > 12288 ? 2 : (groups > 4096 ? 1 : (lz < 4 ? lz : 4));
+    return lz;
 }
 
 // A sum of FP32 terms as hi + lo, or of doubles.
@@ -377,12 +388,11 @@ __global__ void __launch_bounds__(kDiagThreads, kDiagBlocksPerSm)
     diag_kernel(const V2<R> *__restrict__ field, const V4<R> *__restrict__ fluid,
                 LatticeParams<R> P, DiagPartial *__restrict__ partials,
                 unsigned int *__restrict__ ticket, DiagResult *__restrict__ out, const int *__restrict__ status,
-                int *__restrict__ status_out) {
+                int *__restrict__ status_out, int lz) {
     await_previous_launch();
     const uint64_t n = (uint64_t)P.nx * P.ny * P.nz;
     const uint32_t plane = (uint32_t)P.nx * (uint32_t)P.ny;
     const uint32_t groups = (plane + kDiagThreads - 1) / kDiagThreads;
-    const int lz = diag_planes(P.nx, P.ny, P.nz);
     const uint32_t items = groups * (uint32_t)((P.nz + lz - 1) / lz);
     double acc[4] = {0.0, 0.0, 0.0, 0.0};
     R v2max = R(0);
@@ -545,8 +555,7 @@ __global__ void __launch_bounds__(kDiagThreads, kDiagBlocksPerSm)
 }
 
 // One block per item, at most the blocks that `sms` SMs hold.
-inline int diag_blocks(uint64_t nx, uint64_t ny, uint64_t nz, int sms) {
-    const uint64_t lz = (uint64_t)diag_planes(nx, ny, nz);
+inline int diag_blocks(uint64_t nx, uint64_t ny, uint64_t nz, uint64_t lz, int sms) {
     const uint64_t items = (nx * ny + kDiagThreads - 1) / kDiagThreads * ((nz + lz - 1) / lz);
     uint64_t most = (uint64_t)kDiagBlocksPerSm * (uint64_t)(sms > 0 ? sms : 1);
     if (most > (uint64_t)kDiagMaxBlocks) most = kDiagMaxBlocks;

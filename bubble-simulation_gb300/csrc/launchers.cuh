@@ -176,9 +176,10 @@ cudaError_t diag(const V2<R> *field, const V4<R> *fluid, const LatticeParams<R> 
     int device = 0, sms = 0;
     cudaGetDevice(&device);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
-    const int blocks = dev::diag_blocks(P.nx, P.ny, P.nz, sms);
+    const int lz = dev::diag_planes<R, MIXED>(P.nx, P.ny, P.nz);
+    const int blocks = dev::diag_blocks(P.nx, P.ny, P.nz, lz, sms);
     return launch_dependent(dev::diag_kernel<R, MIXED>, dim3((unsigned)blocks), dev::kDiagThreads, 0, s, field, fluid, P,
-                            reinterpret_cast<dev::DiagPartial *>(partials), ticket, out, status, status_out);
+                            reinterpret_cast<dev::DiagPartial *>(partials), ticket, out, status, status_out, lz);
 }
 
 }  // namespace launch_detail
