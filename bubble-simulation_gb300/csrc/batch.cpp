@@ -369,7 +369,8 @@ void Batch::plan_items() {
     if (fill_) {
         std::vector<ChunkPlanGrid> grids;
         for (uint32_t k : item_order_) grids.push_back({lats_[k].grid[0], lats_[k].grid[1], lats_[k].grid[2]});
-        const std::vector<int> lz = balanced_chunks(grids, tx, ty_, fast_ && ty_ == 16, max_grid_, lz_cap_);
+        const std::vector<int> lz = fast_ ? balanced_chunks(grids, tx, ty_, ty_ == 16, max_grid_, lz_cap_)
+                                          : spread_chunks(grids, tx, ty_, max_grid_, lz_cap_);
         for (size_t q = 0; q < lz.size(); ++q) lats_[item_order_[q]].lz = lz[q];
     }
     n_items_ = count_items();

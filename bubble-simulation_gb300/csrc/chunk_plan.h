@@ -14,16 +14,57 @@ struct ChunkPlanGrid {
     uint32_t nx, ny, nz;
 };
 
-// Chunks of the shared lattices for the shortest round.  Equal chunks per
-// lattice, no longer than one cap for the first (largest) lattices and a
-// smaller one for the rest, whose short items fill the round's end; among
-// such plans with caps up to cap_max, the one whose round ends first when its
-// items, each its planes and its warm-up's, are handed out in order to the
-// persistent CTAs as they come free.  Any chunking gives the same bits.  The
-// estimate before, the work spread evenly plus the longest item, counted every
-// round's end as a whole item, so it cut too finely, and knew one cap: 16 short
-// solves of 48^3 .. 128^3 were served in 60.8 ms then, in 57.5 ms now, a light
-// stream of 24 at 9.35 solves/s then, at 10.08 now.
+// Equal chunks no longer than the cap: nz cut into as few as that takes.
+inline int equal_chunk(int nz, int cap) {
+    const int pieces = (nz + cap - 1) / cap;
+    return (nz + pieces - 1) / pieces;
+}
+
+// Chunks of the shared lattices in the strict arithmetic: one cap, the one of
+// least cost, the item-planes (each chunk's planes and 2 of warm-up) spread
+// over the persistent grid plus the longest item.  The IEEE divisions of the
+// strict kernel leave their fast path on a fluid at rest, so items of one
+// length differ up to twofold in time and balanced_chunks, which counts planes,
+// cuts too coarsely: 40 steps of a 128^3 lattice are served in 28.4 ms with
+// these chunks and took 38.6 with balanced_chunks', 16 of 48^3 .. 128^3 in 128 and
+// 143 ms; where a round of balanced_chunks' happens to be one wave of short
+// items it is ahead (96^3 8.3 ms, 9.0 here).  The fast arithmetic has no such
+// path (128^3 8.5 ms with balanced_chunks, 9.0 with these, 96^3 3.9 and 4.5).
+inline std::vector<int> spread_chunks(const std::vector<ChunkPlanGrid> &grids, int tx, int ty, int max_grid, int cap_max) {
+    if (max_grid < 1) max_grid = 1;
+    double best = 1e300;
+    int best_cap = cap_max;
+    for (int cap : {cap_max, 48, 32, 24, 16, 12, 8, 6, 4}) {
+        if (cap > cap_max) continue;
+        double planes = 0.0;
+        int longest = 0;
+        for (const ChunkPlanGrid &g : grids) {
+            const long tiles = (long)((g.nx + tx - 1) / tx) * (long)((g.ny + ty - 1) / ty);
+            const int lz = equal_chunk((int)g.nz, cap);
+            const long chunks = ((long)g.nz + lz - 1) / lz;
+            planes += (double)tiles * (double)(g.nz + 2 * chunks);
+            longest = std::max(longest, lz + 2);
+        }
+        const double cost = planes / (double)max_grid + (double)longest;
+        if (cost < best * (1.0 - 1e-9)) {
+            best = cost;
+            best_cap = cap;
+        }
+    }
+    std::vector<int> lz;
+    for (const ChunkPlanGrid &g : grids) lz.push_back(equal_chunk((int)g.nz, best_cap));
+    return lz;
+}
+
+// Chunks of the shared lattices for the shortest round, in the fast arithmetic.
+// Equal chunks per lattice, no longer than one cap for the first (largest)
+// lattices and a smaller one for the rest, whose short items fill the round's
+// end; among such plans with caps up to cap_max, the one whose round ends first
+// when its items, each its planes and its warm-up's, are handed out in order to
+// the persistent CTAs as they come free.  Any chunking gives the same bits.
+// spread_chunks counts every round's end as a whole item, so it cuts too finely
+// here, and knows one cap: 16 short solves of 48^3 .. 128^3 were served in 60.8 ms
+// with it, in 57.5 ms with this, a light stream of 24 at 9.35 and 10.08 solves/s.
 //
 // It runs at each change of membership, while the GPU waits.  Simulating every
 // plan took 0.1 ms for 16 lattices of different ragged sizes and 1.2 ms for 64
@@ -35,10 +76,6 @@ inline std::vector<int> balanced_chunks(const std::vector<ChunkPlanGrid> &grids,
     if (max_grid < 1) max_grid = 1;
     const double warm_up = pair ? 1.6 : 2.0;  // planes, as in the launch cost models (params.h)
     const size_t n = grids.size();
-    auto lz_of = [](int nz, int cap) {
-        const int pieces = (nz + cap - 1) / cap;
-        return (nz + pieces - 1) / pieces;
-    };
     // tiles and the items of the lattices under each cap
     struct Cut {
         int lz;
@@ -57,7 +94,7 @@ inline std::vector<int> balanced_chunks(const std::vector<ChunkPlanGrid> &grids,
         for (size_t q = 0; q < n; ++q) {
             const ChunkPlanGrid &g = grids[q];
             const long tiles = (long)((g.nx + tx - 1) / tx) * (long)((g.ny + ty - 1) / ty);
-            const int lz = lz_of((int)g.nz, caps[c]);
+            const int lz = equal_chunk((int)g.nz, caps[c]);
             const long k = tiles * (((long)g.nz + lz - 1) / lz);
             cuts[c * n + q] = {lz, k};
             items[c * (n + 1) + q + 1] = items[c * (n + 1) + q] + k;
