@@ -50,7 +50,7 @@ LatticeParams<float> params_of(const bubble_model &m, const uint32_t grid[3]) {
 }
 
 std::mutex g_tune_mu;
-std::map<std::tuple<uint32_t, uint32_t, uint32_t, int, bool>, std::vector<std::pair<int, float>>> g_tune_cache;
+std::map<std::tuple<uint32_t, uint32_t, uint32_t, int, bool, int>, int> g_tune_cache;
 
 constexpr size_t kOffStatus = 64;     // counters at 0 (16 B), status at 64
 constexpr size_t kOffDiag = 256;      // diag partials | ticket
@@ -74,27 +74,20 @@ std::string check_spec(const bubble_spec &s, int math) {
 // ---------------------------------------------------------------------------
 //  Autotuner
 // ---------------------------------------------------------------------------
-// `shortest`: the fewest planes considered; a batch, whose other lattices fill
-// the GPU too, takes 4.
+// `shortest`: the fewest planes considered, 1 or 4; a batch, whose other lattices
+// fill the GPU too, takes 4 and times no others (its creation waits for them: five
+// lattices of 24^3 .. 104^3 38.2 ms, 43.3 with the short ones).
 int autotune_chunk(const uint32_t grid[3], int ty, bool fast, int shortest, std::string &err) {
-    const auto key = std::make_tuple(grid[0], grid[1], grid[2], ty, fast);
     const bool pair = fast && ty == 16;
+    if (!pair) shortest = 4;
+    const auto key = [&](int least) { return std::make_tuple(grid[0], grid[1], grid[2], ty, fast, least); };
     // the chunk that set_tile takes for the pair form's own pick
     const int stands_for_pick = pair ? default_chunk(grid, 16, true) : 0;
     const int pick = pair ? pair_chunk(grid) : 0;
-    const auto best_of = [&](const std::vector<std::pair<int, float>> &timed) {
-        std::pair<int, float> best{0, 1e30f};
-        for (const auto &t : timed) {
-            if (t.first < shortest && t.first < (int)grid[2]) continue;
-            if (shortest == 1 && t.first == stands_for_pick && t.first != pick) continue;
-            if (t.second < best.second) best = t;
-        }
-        return best.first;
-    };
     {
         std::lock_guard<std::mutex> g(g_tune_mu);
-        auto it = g_tune_cache.find(key);
-        if (it != g_tune_cache.end()) return best_of(it->second);
+        auto it = g_tune_cache.find(key(shortest));
+        if (it != g_tune_cache.end()) return it->second;
     }
     bubble_spec spec;
     std::memset(&spec, 0, sizeof(spec));
@@ -117,17 +110,25 @@ int autotune_chunk(const uint32_t grid[3], int ty, bool fast, int shortest, std:
     }
     const int nz = (int)grid[2];
     std::vector<int> cand;
-    // the pair form runs small lattices fastest with chunks below 4 planes
-    // (32^3: 17.2 us per step with 1, 29.9 with 4)
-    if (pair) cand = {1, 2, 3};
     for (int lz : {4, 6, 8, 12, 16, 24, 32, 48, 64, 96, 128, 192, 256})
         if (lz < nz) cand.push_back(lz);
     cand.push_back(nz);
-    if (pair && std::find(cand.begin(), cand.end(), pick) == cand.end()) cand.push_back(pick);
-    std::vector<std::pair<int, float>> timed;
+    const size_t listed = cand.size();
+    // the pair form runs small lattices fastest with chunks below 4 planes
+    // (32^3: 17.2 us per step with 1, 29.9 with 4)
+    if (shortest == 1) {
+        cand.insert(cand.end(), {1, 2, 3});
+        if (std::find(cand.begin(), cand.end(), pick) == cand.end()) cand.push_back(pick);
+    }
+    struct Best {
+        int lz;
+        float ms = 1e30f;
+    };
+    Best any{pick}, four{cand.front()};  // of all of them, of the listed ones
     // The quiescent initial state is an exact fixed point of the scheme, so
     // timing steps on it does not change the lattice.
-    for (int lz : cand) {
+    for (size_t c = 0; c < cand.size(); ++c) {
+        const int lz = cand[c];
         TileShape tile{tile_x_for(ty), ty, lz};
         tile.pair_lz = lz;
         if (sim->set_tile(tile, err) != BUBBLE_OK) continue;
@@ -138,15 +139,15 @@ int autotune_chunk(const uint32_t grid[3], int ty, bool fast, int shortest, std:
         cudaEventSynchronize(e1);
         float ms = 0.0f;
         cudaEventElapsedTime(&ms, e0, e1);
-        timed.emplace_back(lz, ms);
+        if (c < listed && ms < four.ms) four = {lz, ms};
+        if ((lz != stands_for_pick || lz == pick) && ms < any.ms) any = {lz, ms};
     }
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
-    if (timed.empty()) timed.emplace_back(cand.front(), 0.0f);
-    const int best = best_of(timed);
     std::lock_guard<std::mutex> g(g_tune_mu);
-    g_tune_cache[key] = std::move(timed);
-    return best;
+    g_tune_cache[key(4)] = four.lz;
+    if (shortest == 1) g_tune_cache[key(1)] = any.lz;
+    return shortest == 1 ? any.lz : four.lz;
 }
 
 // ---------------------------------------------------------------------------
